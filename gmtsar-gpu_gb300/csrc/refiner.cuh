@@ -10,9 +10,19 @@ namespace xcg {
 // flat parameter vector (FP32): conv weights [c_out][c_in][3][3], dense [out][in]
 constexpr int RP_W1 = 0, RP_B1 = 288, RP_W2 = 320, RP_B2 = 9536, RP_W3 = 9568, RP_B3 = 18784, RP_F1 = 18816,
               RP_C1 = 37248, RP_F2 = 37312, RP_C2 = 37504, RP_N = 37507;
-// per-sample activation record (and the same layout for its gradients)
-constexpr int ACT_Y1 = 0, ACT_A1 = 1568, ACT_Y2 = 3136, ACT_A2 = 3936, ACT_Y3 = 4736, ACT_A3 = 5024, ACT_Z1 = 5312,
-              ACT_G1 = 5376, ACT_OUT = 5440, REF_ACT = 5444;
+// per-sample training records.  Activations as k_ref_fwd holds them in shared
+// memory: 7-wide rows padded to 8 floats with channels A1_CS apart (5-wide:
+// A2_CS), the dense input unpadded; beside each its GELU derivative (rows
+// padded to 8, channels unpadded).  Gradients of the pre-activations: conv1's
+// like the activations, conv2's with channels 40 apart, conv3's in rows of 4
+// with channels 12 apart.  Every section starts on 16 bytes.
+constexpr int A1_CS = 60, A2_CS = 44, A1_LEN = 32 * A1_CS, A2_LEN = 32 * A2_CS;
+constexpr int ACT_A1 = 0, ACT_A2 = ACT_A1 + A1_LEN, ACT_A3 = ACT_A2 + A2_LEN, ACT_G1 = ACT_A3 + 288, ACT_D1 = ACT_G1 + 64,
+              ACT_D2 = ACT_D1 + 32 * 56, ACT_D3 = ACT_D2 + 32 * 40, ACT_DZ = ACT_D3 + 288, ACT_OUT = ACT_DZ + 64,
+              REF_ACT = ACT_OUT + 4;
+constexpr int GRD_Y1 = 0, GRD_Y2 = A1_LEN, GRD_Y3 = GRD_Y2 + 32 * 40, GRD_Z = GRD_Y3 + 32 * 12, GRD_OUT = GRD_Z + 64,
+              REF_GRAD = GRD_OUT + 4;
+constexpr int REF_SMS = 152;         // CTAs of a full training launch: one per SM
 // Inference parameter pack (built by k_ref_derive, copied whole into each
 // inference CTA's shared memory): 128 BF16 weight rows -- conv2 (32), conv3
 // (32), dense 288->64 (64) -- with K reordered tap- (or position-) major,
@@ -27,15 +37,19 @@ constexpr int INF_PACK_BYTES = INF_ROWS * INF_KS * 2 + INF_SMALL * 4;     // 78,
 struct RefPlan {
     float *theta, *m, *v, *grad;        // RP_N each
     float *w2t, *w3t, *f1t;             // transposed FP32 copies (training forward)
+    float *w2b, *w3b;                   // the convolutions' weights as [c_out][tap][c_in] (training backward)
     unsigned char *wpack;               // INF_PACK_BYTES, the inference parameter pack
-    float *act, *grad_act;              // [batch][REF_ACT]
+    float *act, *grad_act;              // [batch][REF_ACT], [batch][REF_GRAD]
+    float *part;                        // [ref_wgrad_parts(batch)][RP_N] partial parameter gradients
     float *loss;                        // [batch] per-sample loss (nullable)
     float *out;                         // [batch][3] training-forward outputs (nullable)
 };
 
 cudaError_t ref_setup();
-void ref_launch_fwd(const RefPlan &R, const float *feat, int n, cudaStream_t s);
+// train: keep what the backward kernels read in the samples' records
+void ref_launch_fwd(const RefPlan &R, const float *feat, int n, bool train, cudaStream_t s);
 void ref_launch_bwd(const RefPlan &R, const float *target, int n, cudaStream_t s);
+int ref_wgrad_parts(int n);
 void ref_launch_wgrad(const RefPlan &R, const float *feat, int n, cudaStream_t s);
 void ref_launch_adam(const RefPlan &R, float lr, int step, cudaStream_t s);
 void ref_launch_derive(const RefPlan &R, cudaStream_t s);

@@ -51,7 +51,8 @@ xcg_status xcg_refiner_create(int32_t device, int32_t max_batch, xcg_refiner **o
     auto take = [&](size_t bytes) { size_t o = off; off += a256(bytes); return o; };
     const size_t o_th = take(np * 4), o_m = take(np * 4), o_v = take(np * 4), o_g = take(np * 4);
     const size_t o_w2t = take(9216 * 4), o_w3t = take(9216 * 4), o_f1t = take(18432 * 4), o_bf = take(xcg::INF_PACK_BYTES);
-    const size_t o_act = take((size_t)max_batch * xcg::REF_ACT * 4), o_gact = take((size_t)max_batch * xcg::REF_ACT * 4);
+    const size_t o_w2b = take(9216 * 4), o_w3b = take(9216 * 4), o_part = take((size_t)xcg::ref_wgrad_parts(max_batch) * np * 4);
+    const size_t o_act = take((size_t)max_batch * xcg::REF_ACT * 4), o_gact = take((size_t)max_batch * xcg::REF_GRAD * 4);
     const size_t o_loss = take((size_t)max_batch * 4), o_out = take((size_t)max_batch * 12);
     xcg_status st = ck(cudaMalloc(&r->mem, off), "cudaMalloc refiner");
     if (st != XCG_OK) { delete r; return st; }
@@ -59,6 +60,7 @@ xcg_status xcg_refiner_create(int32_t device, int32_t max_batch, xcg_refiner **o
     r->R.theta = (float *)(b + o_th); r->R.m = (float *)(b + o_m); r->R.v = (float *)(b + o_v); r->R.grad = (float *)(b + o_g);
     r->R.w2t = (float *)(b + o_w2t); r->R.w3t = (float *)(b + o_w3t); r->R.f1t = (float *)(b + o_f1t);
     r->R.wpack = (unsigned char *)(b + o_bf);
+    r->R.w2b = (float *)(b + o_w2b); r->R.w3b = (float *)(b + o_w3b); r->R.part = (float *)(b + o_part);
     r->R.act = (float *)(b + o_act); r->R.grad_act = (float *)(b + o_gact);
     r->R.loss = (float *)(b + o_loss);
     r->out_int = (float *)(b + o_out);
@@ -109,7 +111,7 @@ xcg_status xcg_refiner_forward(xcg_refiner *r, const float *d_feat, int32_t n, f
             R.out = d_out + (size_t)c0 * 3;
             R.loss = nullptr;
             const int m = (n - c0 < r->max_batch) ? n - c0 : r->max_batch;
-            xcg::ref_launch_fwd(R, d_feat + (size_t)c0 * 81, m, s);
+            xcg::ref_launch_fwd(R, d_feat + (size_t)c0 * 81, m, false, s);
         }
     }
     return ck(cudaGetLastError(), "refiner forward");
@@ -118,7 +120,7 @@ xcg_status xcg_refiner_forward(xcg_refiner *r, const float *d_feat, int32_t n, f
 static void run_grad(xcg_refiner *r, const float *d_feat, const float *d_target, int n, cudaStream_t s) {
     xcg::RefPlan R = r->R;
     R.out = r->out_int;
-    xcg::ref_launch_fwd(R, d_feat, n, s);
+    xcg::ref_launch_fwd(R, d_feat, n, true, s);
     xcg::ref_launch_bwd(R, d_target, n, s);
     xcg::ref_launch_wgrad(R, d_feat, n, s);
 }
