@@ -691,30 +691,34 @@ k_cols_rcp(Plan P) {
     float2 *boxx = boxy + M;                    // [CP + 1] DFT of the column mask at this tile's kx, then N/2
     double *dsum = reinterpret_cast<double *>(boxx + CP + 1);   // [4] per-warp partial chunk sums
     int *grab = reinterpret_cast<int *>(dsum + 4);              // [1] the next chunk of tiles (thread 0's grab)
+    float *mval = reinterpret_cast<float *>(grab + 1);          // [2] the window's master DC term and slave mean
 
     const int N = P.npx, NH = N / 2;
     const int NG = NH / CP;                     // column groups per window
     const int ntiles = P.nwin * NG;
-    // Tiles come in chunks of a quarter window from a counter the planner
-    // zeroed (a CTA that starts late, behind the other batch's kernels, takes
-    // fewer), or, without the counter, as one contiguous range per CTA.
+    // Tiles come in chunks from a counter the planner zeroed (a CTA that
+    // starts late, behind the other batch's kernels, takes fewer), or,
+    // without the counter, as one contiguous range per CTA.  A chunk is a
+    // quarter window, or half of a CTA's even share of the tiles where that is
+    // less: a strip of 20 windows of 128 x 128 (320 tiles) in quarter windows
+    // ran on 80 CTAs, four tiles one after another (86.2 against 73.0 us per
+    // call in single tiles).  Shorter chunks towards the end of a large batch
+    // cost more in patch means than the shorter tail gives (1000 windows of
+    // 128 x 128: 426 against 420 us).
     const bool dyn = (P.rc_tile_next != nullptr);
-    const int K = (NG >= 4) ? NG / 4 : 1;
+    const int K = max(1, min(NG / 4, ntiles / (2 * (int)gridDim.x)));
     int t, tend;                                // the current chunk [t, tend)
     if (dyn) {
         if (threadIdx.x == 0) *grab = atomicAdd(P.rc_tile_next, K);
         __syncthreads();
         t = *grab;
+        tend = min(t + K, ntiles);
         __syncthreads();                        // every thread has read it before the next grab
     } else {
         t = (int)((long long)ntiles * blockIdx.x / gridDim.x);
         tend = (int)((long long)ntiles * (blockIdx.x + 1) / gridDim.x);
-        if (t >= tend) return;
     }
-    if (dyn) {
-        if (t >= ntiles) return;
-        tend = min(t + K, ntiles);
-    }
+    if (t >= tend) return;
     const int warp = threadIdx.x >> 5, l32 = threadIdx.x & 31;
     const int lane = l32 % T;
     const int team = warp * (32 / T) + l32 / T;
@@ -759,7 +763,6 @@ k_cols_rcp(Plan P) {
     for (int i = threadIdx.x; i < M; i += THR) boxy[i] = __ldg(P.box_y + i);
 
     int cur_w = -1;
-    float dc1 = 0.f, m2 = 0.f;
     for (;;) {
         int w, b;
         tile(t, w, b);
@@ -784,14 +787,16 @@ k_cols_rcp(Plan P) {
         int tn = -1;                             // the next tile, none: -1
         if (t + 1 < tend) tn = t + 1;
         else if (dyn && *grab < ntiles) tn = *grab;
-        if (neww) {
+        if (neww && warp == 0) {                 // one warp: GB300 issues two FP64 operations per SM and cycle
             const double inv = pow2_inv(N * M);
             const double s1 = (dsum[0] + dsum[1]) * inv, s2 = (dsum[2] + dsum[3]) * inv;
-            dc1 = (float)(s1 * (double)N * (double)M);
-            m2 = (float)s2;
-            if (b == 0 && threadIdx.x == 0) { P.means[2 * w] = s1; P.means[2 * w + 1] = s2; }
-            cur_w = w;
+            if (l32 == 0) {
+                mval[0] = (float)(s1 * (double)N * (double)M);
+                mval[1] = (float)s2;
+                if (b == 0) { P.means[2 * w] = s1; P.means[2 * w + 1] = s2; }
+            }
         }
+        cur_w = w;
 
         const int kx = kx0 + team;
         float2 *a = cols + team * CS;            // master column, later the result
@@ -813,6 +818,7 @@ k_cols_rcp(Plan P) {
         }
         cp_async_wait<0>();                      // master rows in
         __syncthreads();
+        const float dc1 = mval[0], m2 = mval[1];
 #pragma unroll
         for (int m = 0; m < PER; m++) z[m] = a[fft_pad(lane + T * m)];
         __syncwarp();
