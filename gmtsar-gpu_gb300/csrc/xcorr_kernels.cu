@@ -537,6 +537,8 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
     // [nyc / 2 <= 256] surface sum of each row pair, and its part in the reference's half blocks
     float *rowf = reinterpret_cast<float *>(bc + 4);
     float *rowh = rowf + PEAK_MAX_ROW_PAIRS;
+    __shared__ int scan[2];                               // threads that hold the maximum, its position
+    __shared__ unsigned short holder[NT];
 
     const int w = blockIdx.x;
     const int warp = threadIdx.x >> 5, l32 = threadIdx.x & 31;
@@ -546,7 +548,24 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
     const int M = P.npy, nxc = P.nxc, nyc = P.nyc;
     const float scale = 1.0f / ((float)N * (float)M);
 
+    // A row pair's half spectra are copied into the team's exchange buffer
+    // (free between transforms) while the previous pair's values are still
+    // being reduced, so no registers hold loads in flight; columns kx and
+    // N - kx come from one copy.
+    constexpr int QROW = N / 2 + 2;                       // float2 per row in the buffer, 16-byte rows
+    static_assert(2 * QROW <= PADN, "two half-spectrum rows in the exchange buffer");
+    const float2 *q = P.qspec + (size_t)w * nyc * P.qpitch;
+    auto fetch_pair = [&](int pr) {                       // rows 2 pr and 2 pr + 1
+        const float2 *src = q + (size_t)(2 * pr) * P.qpitch;
+        for (int i = lane; i < QROW; i += T) {            // QROW / 2 16-byte pieces per row
+            const int r = i >= QROW / 2 ? 1 : 0, c = 2 * (i - r * (QROW / 2));
+            cp_async16(ex + r * QROW + c, src + (size_t)r * P.qpitch + c);
+        }
+        cp_async_commit();
+    };
+    if (team < nyc / 2) fetch_pair(team);
     for (int i = threadIdx.x; i < TWL; i += NT) tw[i] = P.tw_row[i];
+    __syncthreads();
     // The reference's surface is exactly zero when either demeaned patch is
     // (its FFTs of zeros stay zeros); the packed transform here would leave
     // rounding residue of the other patch, so that case is set explicitly.
@@ -592,24 +611,32 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
             bc[3] = oobf ? 1.0 : 0.0;
         }
     }
-    __syncthreads();
-    const float keep = (float)bc[2];
-    unsigned long long best = 0ull;
-    const float2 *q = P.qspec + (size_t)w * nyc * P.qpitch;
+    float keep = 0.f;
+    bool synced = false;                                  // bc written by warp 0, seen by all
+    float lmax = 0.f;                                     // the largest value of this thread, if positive
     float *surf = P.surf + (size_t)w * nyc * nxc;
-    for (int pr = team; pr < nyc / 2; pr += teams) {
+    for (int pr = team; pr < nyc / 2; pr += teams) {      // the same trips for every team of a warp
         const int y1 = 2 * pr, y2 = y1 + 1;
         // two real rows in one complex inverse FFT: S = Q1 + i Q2, Hermitian-extended
+        cp_async_wait<0>();
+        __syncwarp();
         float2 v[PER];
 #pragma unroll
         for (int m = 0; m < PER; m++) {
             const int e = lane + T * m;
             const int kx = (e <= N / 2) ? e : N - e;
-            float2 q1 = q[(size_t)y1 * P.qpitch + kx], q2 = q[(size_t)y2 * P.qpitch + kx];
+            float2 q1 = ex[kx], q2 = ex[QROW + kx];
             if (kx == 0 || kx == N / 2) { q1.y = 0.f; q2.y = 0.f; }
             v[m] = (e <= N / 2) ? make_float2(q1.x - q2.y, q1.y + q2.x) : make_float2(q1.x + q2.y, q2.x - q1.y);
         }
+        __syncwarp();
         team_fft_reg<N, +1>(v, ex, tw, lane);
+        if (pr + teams < nyc / 2) fetch_pair(pr + teams);
+        if (!synced) {
+            __syncthreads();
+            keep = (float)bc[2];
+            synced = true;
+        }
         // surface sums: each row pair's in FP32 (the lane's values, then a
         // fixed tree over the team), then the row pairs in double in a fixed
         // order, so the sums do not depend on the launch shape (GB300's FP64
@@ -617,16 +644,13 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
         // 1e-7 relative, is far below what the statistics need)
         float fpart = 0.f, hpart = 0.f;
 #pragma unroll
-        for (int m = 0; m < PER; m++) {
-            const int xq = lane + T * m - P.nx_corr / 2;
-            if (xq < 0 || xq >= nxc) continue;
+        for (int m = PER / 4; m < 3 * PER / 4; m++) {     // the surface's columns: [N/4, 3N/4)
+            const int xq = lane + T * m - N / 4;
             const float c1 = fabsf(v[m].x * scale) * keep, c2 = fabsf(v[m].y * scale) * keep;
             surf[(size_t)y1 * nxc + xq] = c1;
             surf[(size_t)y2 * nxc + xq] = c2;
             const unsigned e1 = (unsigned)(y1 * nxc + xq), e2 = (unsigned)(y2 * nxc + xq);
-            const unsigned long long k1 = argmax_key(c1, e1), k2 = argmax_key(c2, e2);
-            best = k1 > best ? k1 : best;
-            best = k2 > best ? k2 : best;
+            lmax = fmaxf(lmax, fmaxf(c1, c2));
             fpart += c1 + c2;
             if (!(e1 & 512u)) hpart += c1;      // reduce6<double,1024> keeps local [0,512) and [1024,1536)
             if (!(e2 & 512u)) hpart += c2;
@@ -638,24 +662,56 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
         }
         if (lane == 0) { rowf[pr] = fpart; rowh[pr] = hpart; }
     }
-    best = warp_max_u64(best);
-    if (l32 == 0) rk[warp] = best;
+    if (!synced) __syncthreads();                         // a warp without row pairs
+    // The argmax in two phases: the largest value first, then its position
+    // among the threads that hold it (argmax_key's order: the position is the
+    // smallest (block, bit-reversed index) of the elements with that value;
+    // without a positive value it is element 0).  One maximum per element
+    // instead of a 64-bit key (with the copies below: 98 -> 87 us per 1000
+    // windows of 128 x 128).
+    {
+        const unsigned wm = __reduce_max_sync(0xffffffffu, __float_as_uint(lmax));   // non-negative floats order as their bits
+        if (l32 == 0) rk[warp] = wm;
+        if (threadIdx.x == 0) { scan[0] = 0; scan[1] = 0x7fffffff; }
+    }
     __syncthreads();
-    if (warp == 0) {
+    float vmax;
+    {
+        unsigned m = 0;
+#pragma unroll
+        for (int i = 0; i < NW; i++) m = max(m, (unsigned)rk[i]);
+        vmax = __uint_as_float(m);
+    }
+    if (vmax > 0.f && lmax == vmax) holder[atomicAdd(&scan[0], 1)] = (unsigned short)threadIdx.x;
+    if (warp == NW - 1) {
         double hs = 0.0, fs = 0.0;
         for (int i = l32; i < nyc / 2; i += 32) { hs += (double)rowh[i]; fs += (double)rowf[i]; }
         hs = warp_sum_f64(hs);
         fs = warp_sum_f64(fs);
-        if (l32 == 0) {
-            unsigned long long bb = rk[0];
-            for (int i = 1; i < NW; i++) bb = rk[i] > bb ? rk[i] : bb;
-            rk[0] = bb; rd[0] = hs; rd[NW] = fs;
+        if (l32 == 0) { rd[0] = hs; rd[NW] = fs; }
+    }
+    __syncthreads();
+    {
+        // a holder's elements: both rows of its team's row pairs, its lane's columns
+        constexpr int CPL = PER / 2;                      // surface columns per lane
+        const int per = 2 * CPL * ((nyc / 2 + teams - 1) / teams);
+        const int nh = scan[0];
+        for (int i = threadIdx.x; i < nh * per; i += NT) {
+            const int h = i / per, j = i - h * per;
+            const int th = holder[h], hl = (th & 31) % T, ht = (th >> 5) * (32 / T) + (th & 31) / T;
+            const int y = 2 * (ht + (j / (2 * CPL)) * teams) + (j & 1);
+            const int x = hl + T * ((j >> 1) % CPL + PER / 4) - nxc / 2;
+            if (y < nyc) {
+                const unsigned e = (unsigned)(y * nxc + x);
+                if (surf[e] == vmax) atomicMin(&scan[1], (int)(((e >> 11) << 11) | bitrev11(e & 2047u)));
+            }
         }
     }
     __syncthreads();
-    const unsigned pk = argmax_index(rk[0]);
+    const unsigned pos = (vmax > 0.f) ? (unsigned)scan[1] : 0u;
+    const unsigned pk = ((pos >> 11) << 11) | bitrev11(pos & 2047u);
     const int ip = (int)(pk / (unsigned)nxc), jp = (int)(pk % (unsigned)nxc);
-    const double cmax = (double)argmax_value(rk[0]);
+    const double cmax = (double)vmax;
     const float jpeak = (float)jp - (float)nxc / 2.0f;     // do_freq_xcorr.cu:158-159
     const float ipeak = (float)ip - (float)nyc / 2.0f;
 
@@ -677,54 +733,51 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
     }
     long long sn = 0, s1 = 0, s2 = 0;
     constexpr int NXC = N / 2;          // nx_corr = 2 xsearch = npx / 2
-    if constexpr (N <= 256) {
-        // The rows are staged by cp.async in the transforms' exchange buffers,
-        // free from here on: RRM rows of both operands per round, all of them
-        // in flight at once without holding registers (the peak stage of
-        // these sizes is latency-bound: 0.107 -> 0.098 ms per 1000 windows of
-        // 128 x 128; the 512-point stage, at several waves, is faster with the
-        // register loads below).  The sums are integers, so their order does
-        // not change them.
-        constexpr int FBF = (NT / T) * PADN * 2;        // floats of the exchange buffers
-        constexpr int RRM = FBF / (2 * NXC);            // rows of both operands per round
-        static_assert(RRM >= 1 && NXC % 4 == 0, "staging rows");
-        float *sa = reinterpret_cast<float *>(fb), *sb = sa + RRM * NXC;
-        for (int r0 = 0; r0 < P.ny_corr; r0 += RRM) {
-            const int n = min(RRM, P.ny_corr - r0) * NXC;
-            for (int i = threadIdx.x; i < n; i += NT) {      // master rows at the peak offset: any alignment
-                const int r = i / NXC, cc = i - r * NXC;
-                cp_async4(sa + i, a1 + (size_t)(r0 + r) * N + cc);
+    {
+        // The rows come by cp.async through the transforms' exchange buffers,
+        // free from here on, in two halves: one is summed while the other's
+        // copies are in flight.  The master's rows start at any column: their
+        // 16-byte pieces from the column below, one piece more than a row
+        // (columns jp & ~3 .. + NXC + 3 stay inside the N amplitudes of a row).
+        // The sums are integers, so their order does not change them.
+        constexpr int FBF = (NT / T) * PADN * 2;          // floats of the exchange buffers
+        constexpr int SA = NXC + 4;                       // master row in the buffer
+        constexpr int RR = FBF / (2 * (SA + NXC));        // rows of both operands per half
+        static_assert(RR >= 1 && NXC % 4 == 0, "staging rows");
+        float *st = reinterpret_cast<float *>(fb);
+        const int ash = (int)((unsigned)jp & 3u);
+        const float *a1q = a1 - ash;
+        auto stage = [&](int r0, int half) {
+            float *sa = st + half * RR * (SA + NXC), *sb = sa + RR * SA;
+            const int n = min(RR, P.ny_corr - r0);
+            for (int i = threadIdx.x; i < n * (SA / 4); i += NT) {
+                const int r = i / (SA / 4), c = 4 * (i - r * (SA / 4));
+                cp_async16(sa + r * SA + c, a1q + (size_t)(r0 + r) * N + c);
             }
-            for (int i = threadIdx.x; i < n / 4; i += NT) {  // the slave's centre: 16-byte aligned rows
-                const int e = 4 * i, r = e / NXC, cc = e - r * NXC;
-                cp_async16(sb + e, a2 + (size_t)(r0 + r) * a2s + cc);
+            for (int i = threadIdx.x; i < n * (NXC / 4); i += NT) {
+                const int r = i / (NXC / 4), c = 4 * (i - r * (NXC / 4));
+                cp_async16(sb + r * NXC + c, a2 + (size_t)(r0 + r) * a2s + c);
             }
             cp_async_commit();
-            cp_async_wait<0>();
+        };
+        stage(0, 0);
+        for (int r0 = 0, half = 0; r0 < P.ny_corr; r0 += RR, half ^= 1) {
+            if (r0 + RR < P.ny_corr) {
+                stage(r0 + RR, half ^ 1);
+                cp_async_wait<1>();
+            } else {
+                cp_async_wait<0>();
+            }
             __syncthreads();
+            const float *sa = st + half * RR * (SA + NXC) + ash, *sb = st + half * RR * (SA + NXC) + RR * SA;
+            const int n = min(RR, P.ny_corr - r0) * NXC;
+#pragma unroll 4
             for (int i = threadIdx.x; i < n; i += NT) {
-                const long long ia = (long long)(int)(sa[i] - m1f), ib = (long long)(int)(sb[i] - m2f);
-                sn += ia * ib; s1 += ia * ia; s2 += ib * ib;
-            }
-            __syncthreads();             // read before the next round's copies land
-        }
-    } else {
-        constexpr int GU = 8;            // loads in flight per thread and operand
-        const int ntot = P.ny_corr * NXC;   // a multiple of NT * GU
-        for (int i0 = threadIdx.x; i0 < ntot; i0 += NT * GU) {
-            float va[GU], vb[GU];
-#pragma unroll
-            for (int u = 0; u < GU; u++) {
-                const int i = i0 + u * NT;
                 const int r = i / NXC, cc = i - r * NXC;
-                va[u] = __ldg(a1 + (size_t)r * N + cc);
-                vb[u] = __ldg(a2 + (size_t)r * a2s + cc);
-            }
-#pragma unroll
-            for (int u = 0; u < GU; u++) {
-                const long long ia = (long long)(int)(va[u] - m1f), ib = (long long)(int)(vb[u] - m2f);
+                const long long ia = (long long)(int)(sa[r * SA + cc] - m1f), ib = (long long)(int)(sb[i] - m2f);
                 sn += ia * ib; s1 += ia * ia; s2 += ib * ib;
             }
+            __syncthreads();             // read before the copies after the next land
         }
     }
     sn = warp_sum_i64(sn); s1 = warp_sum_i64(s1); s2 = warp_sum_i64(s2);
