@@ -34,54 +34,17 @@ namespace xcg {
 
 __device__ __forceinline__ unsigned bitrev11(unsigned e) { return __brev(e) >> 21; }
 
-// Sortable argmax key with the reference's tie rules (reduce6b / reduce6bC,
-// conv_ampl_demean.cu:227-346,434-554, host finish :655-673,739-754): a
-// thread starts from value 0 at the first element of its pair and takes a
-// later element only if strictly greater; tree levels keep the lower thread
-// on ties; the host keeps the earliest block.  Net effect: the winner has the
-// largest effective value, ties to the smallest (block, bit-reversed local
-// index); an element that is not > 0 counts as 0 in the first half of its
-// 2048-element block and never wins in the second half.
-__device__ __forceinline__ unsigned long long argmax_key(float v, unsigned e) {
-    const unsigned local = e & 2047u;
-    unsigned ord;
-    if (v > 0.f) ord = __float_as_uint(v) + 1u;
-    else ord = (local < 1024u) ? 1u : 0u;          // 0.0f -> 1, "never" -> 0
-    const unsigned key = ((e >> 11) << 11) | bitrev11(local);
-    return ((unsigned long long)ord << 32) | (0xffffffffu - key);
-}
-__device__ __forceinline__ unsigned argmax_index(unsigned long long k) {
-    const unsigned key = 0xffffffffu - (unsigned)(k & 0xffffffffu);
-    return ((key >> 11) << 11) | bitrev11(key & 2047u);
-}
-__device__ __forceinline__ float argmax_value(unsigned long long k) {
-    const unsigned ord = (unsigned)(k >> 32);
-    return ord <= 1u ? 0.f : __uint_as_float(ord - 1u);
-}
+// Position order of the argmax with the reference's tie rules (reduce6b /
+// reduce6bC, conv_ampl_demean.cu:227-346,434-554, host finish
+// :655-673,739-754): a thread starts from value 0 at the first element of its
+// pair and takes a later element only if strictly greater; tree levels keep
+// the lower thread on ties; the host keeps the earliest block.  Net effect: the
+// winner has the largest value, ties to the smallest (2048-element block,
+// bit-reversed local index); an element that is not > 0 counts as 0 in the
+// first half of its block and never wins in the second half, so without a
+// positive element it is element 0 with value 0.
+__device__ __forceinline__ unsigned argmax_order(unsigned e) { return (e & ~2047u) | bitrev11(e & 2047u); }   // its own inverse
 
-// best = max(best, argmax_key(v, e)), the key built only where it can win.
-// Keys order by their value word first, and every positive value's word
-// (its bits + 1) is above the words of zero, negative and NaN values (0 or 1),
-// so once best holds a positive value, a value below it cannot win; bestv is
-// that value, or -inf while best holds none (then every key is built).
-__device__ __forceinline__ void argmax_update(unsigned long long &best, float &bestv, float v, unsigned e) {
-    if (!(v < bestv)) {
-        const unsigned long long k = argmax_key(v, e);
-        if (k > best) {
-            best = k;
-            bestv = ((unsigned)(k >> 32) >= 2u) ? argmax_value(k) : -INFINITY;
-        }
-    }
-}
-
-__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        unsigned long long u = __shfl_xor_sync(0xffffffffu, v, o);
-        v = u > v ? u : v;
-    }
-    return v;
-}
 __device__ __forceinline__ long long warp_sum_i64(long long v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -664,9 +627,8 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
     }
     if (!synced) __syncthreads();                         // a warp without row pairs
     // The argmax in two phases: the largest value first, then its position
-    // among the threads that hold it (argmax_key's order: the position is the
-    // smallest (block, bit-reversed index) of the elements with that value;
-    // without a positive value it is element 0).  One maximum per element
+    // among the threads that hold it (the smallest argmax_order of the elements
+    // with that value; element 0 without a positive value).  One maximum per element
     // instead of a 64-bit key (with the copies below: 98 -> 87 us per 1000
     // windows of 128 x 128).
     {
@@ -703,13 +665,13 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
             const int x = hl + T * ((j >> 1) % CPL + PER / 4) - nxc / 2;
             if (y < nyc) {
                 const unsigned e = (unsigned)(y * nxc + x);
-                if (surf[e] == vmax) atomicMin(&scan[1], (int)(((e >> 11) << 11) | bitrev11(e & 2047u)));
+                if (surf[e] == vmax) atomicMin(&scan[1], (int)argmax_order(e));
             }
         }
     }
     __syncthreads();
     const unsigned pos = (vmax > 0.f) ? (unsigned)scan[1] : 0u;
-    const unsigned pk = ((pos >> 11) << 11) | bitrev11(pos & 2047u);
+    const unsigned pk = argmax_order(pos);
     const int ip = (int)(pk / (unsigned)nxc), jp = (int)(pk % (unsigned)nxc);
     const double cmax = (double)vmax;
     const float jpeak = (float)jp - (float)nxc / 2.0f;     // do_freq_xcorr.cu:158-159
@@ -857,24 +819,42 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
 // FFT-pad-IFFT-scale operators, then the argmax of the real part
 // (h_reduceCr_strip, conv_ampl_demean.cu:730-756) and the fractions
 // (highres_corr.cu:59-76).
-__global__ void __launch_bounds__(256) k_subpix(Plan P) {
+// What bounds it: multiply-adds and shared reads of the column pass at eight
+// warps per window.  The row operator stays in registers (a thread's outputs
+// share one column X), the column operator is copied while the neighbourhood
+// is read, and the argmax keeps one maximum per eight values; its position is
+// found afterwards from the group that holds it (a key per value that could
+// win: 48 against 33 us per 1000 windows, 14.3 against 8.2 us for 20).
+template <int IFC>
+__global__ void __launch_bounds__(256, 4) k_subpix(Plan P) {
+    constexpr int N2 = 8, NX2 = N2 * IFC, NT = 256;
+    constexpr int HALF = NX2 / 2;                     // threads per output row: columns X and X + HALF each
+    constexpr int RP = NT / HALF;                     // output rows in flight per pass
+    constexpr int XT = NX2 > NT ? NX2 / NT : 1;       // columns of the row pass per thread
+    constexpr int RT = NX2 > NT ? N2 : N2 * NX2 / NT; // rows of the row pass per thread and column
     extern __shared__ float4 smem_raw[];
-    const int n2x = P.n2x, n2y = P.n2y, nx2 = P.nx2, ny2 = P.ny2;
-    float *md = reinterpret_cast<float *>(smem_raw);                 // [n2y*n2x]
-    float2 *tr = reinterpret_cast<float2 *>(md + 64);                // [n2y][nx2]
-    float2 *kys = tr + n2y * nx2;                                    // [ny2][n2y]
-    float2 *kxs = kys + ny2 * n2y;                                   // [n2x][nx2], transposed
-    unsigned long long *rk = reinterpret_cast<unsigned long long *>(kxs + nx2 * n2x);
-    int *fl = reinterpret_cast<int *>(rk + 8);
+    float *md = reinterpret_cast<float *>(smem_raw);                 // [8][8]
+    float2 *tr = reinterpret_cast<float2 *>(md + 64);                // [8][NX2]
+    float2 *kys = tr + N2 * NX2;                                     // [NX2][8]
+    __shared__ unsigned wmax[NT / 32];
+    __shared__ int scan[2];                                          // threads that hold the maximum, its position
+    __shared__ int holder[NT];
 
-    const int w = blockIdx.x;
+    const int w = blockIdx.x, tid = threadIdx.x;
     if (P.skip && P.skip[w]) return;                  // the refiner answered for this window
-    const int n2 = n2x * n2y;
-    if (threadIdx.x == 0) *fl = 0;
-    __syncthreads();
-    for (int t = threadIdx.x; t < n2; t += blockDim.x) {
-        float v = P.md[(size_t)w * n2 + t];
-        if (P.mdnext[(size_t)w * n2 + t]) {
+    for (int t = tid; t < NX2 * N2 / 2; t += NT) cp_async16(kys + 2 * t, P.ky + 2 * t);
+    cp_async_commit();
+    float4 kx[XT][4];                                 // two entries of the row operator's row X per vector
+#pragma unroll
+    for (int x = 0; x < XT; x++)
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            kx[x][c] = __ldg(reinterpret_cast<const float4 *>(P.kx) + ((tid + x * NT) % NX2) * 4 + c);
+    if (tid == 0) { scan[0] = 0; scan[1] = 0x7fffffff; }
+    int next = 0;
+    if (tid < 64) {
+        float v = P.md[(size_t)w * 64 + tid];
+        if (P.mdnext[(size_t)w * 64 + tid]) {
             // the reference reads the next window of its strip (conv_ampl_demean.cu:84-89)
             int local, pidx, nlocal = -1, npidx = -1;
             const PairDev pd = pair_of(P, w, local, pidx);
@@ -885,50 +865,49 @@ __global__ void __launch_bounds__(256) k_subpix(Plan P) {
             const int g = local + 1;
             const bool same = pd.strip_len > 0 && g < pd.nlocs && (g % pd.strip_len) != 0 && nlocal == g;
             v = same ? powf((float)P.corr0n[w + 1], 0.25f) : 0.f;
-            atomicOr(fl, XCG_FLAG_NEXTREAD);
+            next = 1;
         }
-        md[t] = v;
+        md[tid] = v;
     }
-    for (int t = threadIdx.x; t < ny2 * n2y; t += blockDim.x) kys[t] = __ldg(P.ky + t);
-    for (int t = threadIdx.x; t < nx2 * n2x; t += blockDim.x) {
-        const int X = t / n2x, c = t - X * n2x;
-        kxs[c * nx2 + X] = __ldg(P.kx + t);
-    }
-    __syncthreads();
+    next = __syncthreads_or(next);
     // row pass: tr[r][X] = sum_c md[r][c] * KX[X][c]
-    for (int t = threadIdx.x; t < n2y * nx2; t += blockDim.x) {
-        const int r = t / nx2, X = t - r * nx2;
-        float2 s = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int c = 0; c < 8; c++) {
-            const float2 k = kxs[c * nx2 + X];
-            const float m = md[r * 8 + c];
-            s.x = fmaf(m, k.x, s.x);
-            s.y = fmaf(m, k.y, s.y);
+    for (int x = 0; x < XT; x++)
+#pragma unroll
+        for (int k = 0; k < RT; k++) {
+            const int X = (tid + x * NT) % NX2, r = (NX2 > NT) ? k : tid / NX2 + k * (NT / NX2);
+            const float4 m0 = *reinterpret_cast<const float4 *>(md + r * 8), m1 = *reinterpret_cast<const float4 *>(md + r * 8 + 4);
+            const float m[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+            float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                s.x = fmaf(m[2 * c], kx[x][c].x, s.x);
+                s.y = fmaf(m[2 * c], kx[x][c].y, s.y);
+                s.x = fmaf(m[2 * c + 1], kx[x][c].z, s.x);
+                s.y = fmaf(m[2 * c + 1], kx[x][c].w, s.y);
+            }
+            tr[r * NX2 + X] = s;
         }
-        tr[t] = s;
-    }
+    cp_async_wait<0>();
     __syncthreads();
-    // column pass, real part only, and the argmax: a thread keeps two columns
-    // (X and X + nx2/2) of the row-pass result in registers (2 x n2y values)
-    // and walks the output rows Y, four at a time; a warp shares Y, so each
-    // KY read is one broadcast that feeds both columns
-    unsigned long long best = 0ull;
-    float bestv = -INFINITY;
-    const int half = nx2 / 2;
-    const int tpr = half < (int)blockDim.x ? half : (int)blockDim.x;   // threads per output row
-    const int rp = (int)blockDim.x / tpr;                               // rows in flight per pass
+    // column pass, real part only: a thread keeps two columns (X and X +
+    // NX2/2) of the row-pass result in registers and walks the output rows Y,
+    // four at a time; a warp shares Y, so each KY read is one broadcast that
+    // feeds both columns
     const float4 *ky4 = reinterpret_cast<const float4 *>(kys);          // two KY entries per load
-    for (int X = threadIdx.x % tpr; X < half; X += tpr) {
+    const int X = tid % HALF, Y0 = tid / HALF;
+    float lmax = 0.f;                                 // the largest value of this thread, if positive,
+    int lY = Y0;                                      // the group of rows that holds it first,
+    bool more = false;                                // and whether another group equals it
+    {
         float2 tc[2][8];
 #pragma unroll
-        for (int r = 0; r < 8; r++) { tc[0][r] = tr[r * nx2 + X]; tc[1][r] = tr[r * nx2 + X + half]; }
-        for (int Y = threadIdx.x / tpr; Y < ny2; Y += 4 * rp) {
+        for (int r = 0; r < 8; r++) { tc[0][r] = tr[r * NX2 + X]; tc[1][r] = tr[r * NX2 + X + HALF]; }
+        for (int Y = Y0; Y < NX2; Y += 4 * RP) {
             float re[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const int yy = Y + j * rp;
-                if (yy >= ny2) break;
+                const int yy = Y + j * RP;
 #pragma unroll
                 for (int r2 = 0; r2 < 4; r2++) {
                     const float4 k = ky4[yy * 4 + r2];
@@ -941,37 +920,61 @@ __global__ void __launch_bounds__(256) k_subpix(Plan P) {
                     }
                 }
             }
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int yy = Y + j * rp;
-                if (yy >= ny2) break;
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    argmax_update(best, bestv, re[h][j], (unsigned)(yy * nx2 + X + h * half));
-                }
-            }
+            const float m = fmaxf(fmaxf(fmaxf(re[0][0], re[0][1]), fmaxf(re[0][2], re[0][3])),
+                                  fmaxf(fmaxf(re[1][0], re[1][1]), fmaxf(re[1][2], re[1][3])));
+            more = (m > lmax) ? false : (more || m == lmax);
+            if (m > lmax) { lmax = m; lY = Y; }
         }
     }
-    best = warp_max_u64(best);
-    const int warp = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) rk[warp] = best;
+    {
+        const unsigned wm = __reduce_max_sync(0xffffffffu, __float_as_uint(lmax));   // non-negative floats order as their bits
+        if ((tid & 31) == 0) wmax[tid >> 5] = wm;
+    }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long bb = rk[0];
-        for (int i = 1; i < (int)(blockDim.x >> 5); i++) bb = rk[i] > bb ? rk[i] : bb;
-        const unsigned pk = argmax_index(bb);
-        const int fip = (int)(pk / (unsigned)nx2), fjp = (int)(pk % (unsigned)nx2);
+    unsigned vb = 0;
+#pragma unroll
+    for (int i = 0; i < NT / 32; i++) vb = max(vb, wmax[i]);
+    const float vmax = __uint_as_float(vb);
+    // the position: the smallest argmax_order of the elements with the largest
+    // value (element 0 without a positive one)
+    if (vmax > 0.f && lmax == vmax) holder[atomicAdd(&scan[0], 1)] = tid | (lY << 8) | (more ? 1 << 30 : 0);
+    __syncthreads();
+    for (int i = 0; i < scan[0]; i++) {
+        const int hd = holder[i], ht = hd & 255, hx = ht % HALF;
+        const bool all = (hd >> 30) != 0;
+        const int yb = all ? ht / HALF : (hd >> 8) & 0x3fff, rows = all ? NX2 / RP : 4;   // rows yb, yb + RP, ...
+        for (int j = tid; j < 2 * rows; j += NT) {
+            const int yy = yb + (j >> 1) * RP, xx = hx + (j & 1) * HALF;
+            float re = 0.f;
+#pragma unroll
+            for (int r2 = 0; r2 < 4; r2++) {
+                const float4 k = ky4[yy * 4 + r2];
+                const float2 t0 = tr[2 * r2 * NX2 + xx], t1 = tr[(2 * r2 + 1) * NX2 + xx];
+                re = fmaf(k.x, t0.x, re);
+                re = fmaf(-k.y, t0.y, re);
+                re = fmaf(k.z, t1.x, re);
+                re = fmaf(-k.w, t1.y, re);
+            }
+            const unsigned e = (unsigned)(yy * NX2 + xx);
+            if (re == vmax) atomicMin(&scan[1], (int)argmax_order(e));
+        }
+    }
+    __syncthreads();
+    if (tid == 0) {
+        const unsigned pos = (vmax > 0.f) ? (unsigned)scan[1] : 0u;
+        const unsigned pk = argmax_order(pos);
+        const int fip = (int)(pk / (unsigned)NX2), fjp = (int)(pk % (unsigned)NX2);
         int local, pidx;
         const PairDev pd = pair_of(P, w, local, pidx);
         xcg_result &o = pd.out[local];
         o.fip = fip;
         o.fjp = fjp;
-        o.fmax = argmax_value(bb);
-        const float jpeak = (float)fjp - (float)ny2 / 2.0f;    // ny2 for both axes (highres_corr.cu:61-62)
-        const float ipeak = (float)fip - (float)ny2 / 2.0f;
-        o.xfrac = jpeak / (float)P.ifc;
-        o.yfrac = ipeak / (float)P.ifc;
-        o.flags |= *fl;
+        o.fmax = vmax;
+        const float jpeak = (float)fjp - (float)NX2 / 2.0f;    // ny2 for both axes (highres_corr.cu:61-62)
+        const float ipeak = (float)fip - (float)NX2 / 2.0f;
+        o.xfrac = jpeak / (float)IFC;
+        o.yfrac = ipeak / (float)IFC;
+        if (next) o.flags |= XCG_FLAG_NEXTREAD;
     }
 }
 
@@ -1039,9 +1042,9 @@ template <int N>
 constexpr bool peak_wide_ok() { return N <= 512; }
 template <int N>
 constexpr int peak_wide_minb() { return N <= 256 ? 2 : 1; }
-static size_t subpix_smem(const Plan &P) {
-    return 64 * sizeof(float) + (size_t)P.n2y * P.nx2 * sizeof(float2) + (size_t)P.ny2 * P.n2y * sizeof(float2) +
-           (size_t)P.nx2 * P.n2x * sizeof(float2) + 8 * sizeof(unsigned long long) + 16;
+template <int IFC>
+static size_t subpix_smem() {
+    return 64 * sizeof(float) + (size_t)2 * 8 * 8 * IFC * sizeof(float2);
 }
 
 template <int N>
@@ -1098,10 +1101,8 @@ cudaError_t kernels_setup(const Plan &P) {
         default: return cudaErrorInvalidValue;
     }
     if (e) return e;
-    Plan big = P;                      // the largest interpolated grid any context uses (factor 64)
-    big.nx2 = big.n2x * 64;
-    big.ny2 = big.n2y * 64;
-    return cudaFuncSetAttribute(k_subpix, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)subpix_smem(big));
+    // the interpolated grids beyond the default 48 KB
+    return cudaFuncSetAttribute(k_subpix<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)subpix_smem<64>());
 }
 
 template <int N>
@@ -1167,7 +1168,12 @@ void launch_peak(const Plan &P, cudaStream_t s) {
     }
 }
 void launch_subpix(const Plan &P, cudaStream_t s) {
-    k_subpix<<<P.nwin, 256, subpix_smem(P), s>>>(P);
+    switch (P.ifc) {
+        case 8: k_subpix<8><<<P.nwin, 256, subpix_smem<8>(), s>>>(P); break;
+        case 16: k_subpix<16><<<P.nwin, 256, subpix_smem<16>(), s>>>(P); break;
+        case 32: k_subpix<32><<<P.nwin, 256, subpix_smem<32>(), s>>>(P); break;
+        case 64: k_subpix<64><<<P.nwin, 256, subpix_smem<64>(), s>>>(P); break;
+    }
 }
 
 }  // namespace xcg
