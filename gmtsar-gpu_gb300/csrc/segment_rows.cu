@@ -47,8 +47,6 @@ namespace xcg {
 // ------------------------------------------------------------------ planner
 
 constexpr int RC_ENTRIES = 2 * RC_MAX_WINDOWS;   // sort capacity, a power of two
-constexpr int PLAN_THREADS = 1024;
-constexpr int PER_THREAD = RC_ENTRIES / PLAN_THREADS;
 // Sort key: pair (15 bits) | image (1) | first column + 2^19 (20) | first row
 // modulo the chunk rows (4) | first row + 2^23 (24).  The group of an entry is
 // the key without its low 24 bits.
@@ -56,11 +54,12 @@ constexpr int KEY_Y_BITS = 24;
 constexpr int KEY_Y_BIAS = 1 << 23;
 constexpr int KEY_X_BIAS = 1 << 19;
 
-// In-place exclusive scan of a[0, ns) by the whole CTA (ns a multiple of
-// PLAN_THREADS up to RC_ENTRIES); returns the total.
+// In-place exclusive scan of a[0, ns) by the whole CTA (ns a multiple of NT,
+// at most PER_THREAD of them); returns the total.
+template <int NT, int PER_THREAD>
 __device__ int block_exclusive_scan(int *a, int *wsum, int ns) {
     const int t = threadIdx.x, l32 = t & 31, wp = t >> 5;
-    const int per = ns / PLAN_THREADS;
+    const int per = ns / NT;
     int v[PER_THREAD];
     int s = 0;
 #pragma unroll
@@ -74,7 +73,7 @@ __device__ int block_exclusive_scan(int *a, int *wsum, int ns) {
     if (l32 == 31) wsum[wp] = inc;
     __syncthreads();
     if (wp == 0) {
-        int x = (l32 < PLAN_THREADS / 32) ? wsum[l32] : 0;
+        int x = (l32 < NT / 32) ? wsum[l32] : 0;
         int xi = x;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -98,16 +97,30 @@ __device__ __forceinline__ int key_y(unsigned long long k) {
     return (int)(k & ((1ull << KEY_Y_BITS) - 1)) - KEY_Y_BIAS;
 }
 
-__global__ void __launch_bounds__(PLAN_THREADS, 1) k_rc_plan(Plan P) {
-    extern __shared__ unsigned long long plan_smem[];
-    unsigned long long *key = plan_smem;                        // [RC_ENTRIES] sort keys
-    int *pay = reinterpret_cast<int *>(key + RC_ENTRIES);      // [RC_ENTRIES] entry = 2 w + image
-    int *cnt = pay + RC_ENTRIES;                               // [RC_ENTRIES] run starts before each entry
-    int *rlen = cnt + RC_ENTRIES;                              // [RC_ENTRIES] chunks of each run, then its first chunk
-    int *rhead = rlen + RC_ENTRIES;                            // [RC_ENTRIES] first entry of each run
-    int *rtail = rhead + RC_ENTRIES;                           // [RC_ENTRIES] last entry of each run
-    int *wsum = rtail + RC_ENTRIES;                            // [72] scan scratch
+// One ascending sort of 32 (key, payload) pairs across a warp.
+__device__ __forceinline__ void warp_sort(unsigned long long &k, int &p) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int kk = 2; kk <= 32; kk <<= 1)
+#pragma unroll
+        for (int j = kk >> 1; j > 0; j >>= 1) {
+            const unsigned long long ok = __shfl_xor_sync(0xffffffffu, k, j);
+            const int op = __shfl_xor_sync(0xffffffffu, p, j);
+            const bool small = ((lane & j) == 0) == ((lane & kk) == 0);     // this lane keeps the smaller key
+            if (small ? ok < k : ok > k) { k = ok; p = op; }
+        }
+}
 
+// Latency bounds the planner (one SM per image), so its sort has few
+// barriers: each warp sorts 32 entries by shuffles, then runs are merged by
+// rank, an entry's place being its index in its run plus the entries of the
+// sibling run before it (a binary search), two barriers a level.  Two batches
+// of 500 windows: 32 us of planners with their launches, 41 us with a bitonic
+// network and a barrier per step.  CTAs are as small as the entries allow.
+// (Chunk descriptors of 8 bytes instead of 16 save 1 us more here and cost the
+// row stage 1.6%, unpacking them.)
+template <int NT, int PER>
+__global__ void __launch_bounds__(NT, 1) k_rc_plan(Plan P) {
     const int tid = threadIdx.x;
     // Two CTAs (no row bands): CTA i plans image i's entries alone, its runs
     // never meeting the other image's, and numbers its chunks from
@@ -118,9 +131,20 @@ __global__ void __launch_bounds__(PLAN_THREADS, 1) k_rc_plan(Plan P) {
     const int cbase = (split && blockIdx.x == 1) ? P.nwin * P.nchunks : 0;
     const int npx = P.npx, npy = P.npy, rpc = P.rpc;
     int n = 2;
-    while (n < nent) n <<= 1;
-    const int ns = n > PLAN_THREADS ? n : PLAN_THREADS;   // the entries the loops and scans cover
-    for (int e = tid; e < ns; e += PLAN_THREADS) {
+    while (n < nent || n < 32) n <<= 1;
+    const int ns = n > NT ? n : NT;               // the entries the loops and scans cover
+    extern __shared__ unsigned long long plan_smem[];
+    unsigned long long *key = plan_smem;          // [ns] sort keys
+    int *pay = reinterpret_cast<int *>(key + ns); // [ns] entry = 2 w + image
+    int *cnt = pay + ns;                          // [ns] run starts before each entry
+    int *rlen = cnt + ns;                         // [ns] chunks of each run, then its first chunk
+    int *rhead = rlen + ns;                       // [ns] first entry of each run
+    int *rtail = rhead + ns;                      // [ns] last entry of each run
+    int *wsum = rtail + ns;                       // [72] scan scratch
+#pragma unroll
+    for (int q = 0; q < PER; q++) {
+        const int e = tid + q * NT;
+        if (e >= ns) continue;                    // warp-uniform: ns is a multiple of 32
         unsigned long long k = ~0ull;             // padding sorts last
         const int ge = split ? 2 * e + (int)blockIdx.x : e;    // the entry: 2 w + image
         if (e < nent) {
@@ -135,36 +159,50 @@ __global__ void __launch_bounds__(PLAN_THREADS, 1) k_rc_plan(Plan P) {
                 ((unsigned long long)(x0 + KEY_X_BIAS) << 28) | ((unsigned long long)ym << KEY_Y_BITS) |
                 (unsigned long long)(y0 + KEY_Y_BIAS);
         }
+        int pe = ge;
+        warp_sort(k, pe);
         key[e] = k;
-        pay[e] = ge;
+        pay[e] = pe;
         rlen[e] = 0;
     }
     __syncthreads();
-    // bitonic sort of the first n keys, payload alongside
-    for (int kk = 2; kk <= n; kk <<= 1) {
-        for (int j = kk >> 1; j > 0; j >>= 1) {
-            for (int i = tid; i < n; i += PLAN_THREADS) {
-                const int ixj = i ^ j;
-                if (ixj > i) {
-                    const unsigned long long a = key[i], b = key[ixj];
-                    const bool up = (i & kk) == 0;
-                    if ((a > b) == up) {
-                        key[i] = b; key[ixj] = a;
-                        const int t = pay[i]; pay[i] = pay[ixj]; pay[ixj] = t;
-                    }
-                }
+    for (int len = 32; len < n; len <<= 1) {      // runs of len into runs of 2 len
+        unsigned long long k[PER];
+        int pe[PER], at[PER];
+#pragma unroll
+        for (int q = 0; q < PER; q++) at[q] = -1;      // none: beyond the n entries
+#pragma unroll
+        for (int q = 0; q < PER; q++) {
+            const int e = tid + q * NT;
+            if (e >= n) continue;
+            k[q] = key[e];
+            pe[q] = pay[e];
+            const int run = e / len;
+            const bool left = (run & 1) == 0;     // equal keys: the left run's first
+            const unsigned long long *sib = key + (run ^ 1) * len;
+            int c = 0;
+            for (int h = len >> 1; h > 0; h >>= 1) {
+                const unsigned long long o = sib[c + h - 1];
+                if (left ? o < k[q] : o <= k[q]) c += h;
             }
-            __syncthreads();
+            const unsigned long long o = sib[c];
+            if (left ? o < k[q] : o <= k[q]) c++;
+            at[q] = (run & ~1) * len + (e & (len - 1)) + c;
         }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < PER; q++)
+            if (at[q] >= 0) { key[at[q]] = k[q]; pay[at[q]] = pe[q]; }
+        __syncthreads();
     }
     // a run starts where the group changes or the next patch leaves a gap of rows
     auto is_head = [&](int i) {
         return i == 0 || (key[i] >> KEY_Y_BITS) != (key[i - 1] >> KEY_Y_BITS) || key_y(key[i]) > key_y(key[i - 1]) + npy;
     };
-    for (int i = tid; i < ns; i += PLAN_THREADS) cnt[i] = (i < nent && is_head(i)) ? 1 : 0;
+    for (int i = tid; i < ns; i += NT) cnt[i] = (i < nent && is_head(i)) ? 1 : 0;
     __syncthreads();
-    const int nruns = block_exclusive_scan(cnt, wsum, ns);
-    for (int i = tid; i < nent; i += PLAN_THREADS) {
+    const int nruns = block_exclusive_scan<NT, PER>(cnt, wsum, ns);
+    for (int i = tid; i < nent; i += NT) {
         const bool h = is_head(i);
         const int r = cnt[i] + (h ? 0 : -1);
         if (h) rhead[r] = i;
@@ -172,11 +210,11 @@ __global__ void __launch_bounds__(PLAN_THREADS, 1) k_rc_plan(Plan P) {
     }
     __syncthreads();
     // every patch spans npy rows, so a run ends npy rows below its last entry's first row
-    for (int r = tid; r < nruns; r += PLAN_THREADS)
+    for (int r = tid; r < nruns; r += NT)
         rlen[r] = (key_y(key[rtail[r]]) - key_y(key[rhead[r]]) + npy) / rpc;
     __syncthreads();
-    const int total = block_exclusive_scan(rlen, wsum, ns);   // rlen[r] <- first chunk of run r
-    for (int i = tid; i < nent; i += PLAN_THREADS) {
+    const int total = block_exclusive_scan<NT, PER>(rlen, wsum, ns);   // rlen[r] <- first chunk of run r
+    for (int i = tid; i < nent; i += NT) {
         const int r = cnt[i] + (is_head(i) ? 0 : -1);
         const int c0 = rlen[r] + (key_y(key[i]) - key_y(key[rhead[r]])) / rpc;
         reinterpret_cast<int *>(P.rc_wch)[pay[i]] = cbase + c0;   // rc_wch[w].x for the master, .y for the slave
@@ -184,7 +222,7 @@ __global__ void __launch_bounds__(PLAN_THREADS, 1) k_rc_plan(Plan P) {
     // chunk descriptors: one warp per run, its lanes writing consecutive chunks
     {
         const int wp = tid >> 5, l32 = tid & 31;
-        for (int r = wp; r < nruns; r += PLAN_THREADS / 32) {
+        for (int r = wp; r < nruns; r += NT / 32) {
             const unsigned long long k = key[rhead[r]];
             const int pidx = (int)(k >> 49), img = (int)((k >> 48) & 1);
             const int x0 = (int)((k >> 28) & ((1u << 20) - 1)) - KEY_X_BIAS;
@@ -224,7 +262,7 @@ __global__ void __launch_bounds__(PLAN_THREADS, 1) k_rc_plan(Plan P) {
             return (int)(k < len ? k : len);
         };
         for (int pass = 0; pass < 2; pass++) {
-            for (int r = wp; r < nruns; r += PLAN_THREADS / 32) {
+            for (int r = wp; r < nruns; r += NT / 32) {
                 const unsigned long long k = key[rhead[r]];
                 const int img = (int)((k >> 48) & 1), y0 = key_y(k);
                 const int c0 = rlen[r], len = ((r + 1 < nruns) ? rlen[r + 1] : total) - c0;
@@ -914,8 +952,13 @@ k_cols_rcp(Plan P) {
 
 // ------------------------------------------------------------------ launchers
 
-static size_t rc_plan_smem_bytes() {
-    return (size_t)RC_ENTRIES * (sizeof(unsigned long long) + 5 * sizeof(int)) + 72 * sizeof(int);
+// threads of the planner for nent entries per CTA: one entry each up to 512,
+// then up to eight (a CTA of 1024 threads waits for an SM without other work)
+static int plan_threads(int nent) { return nent <= 128 ? 128 : 512; }
+static size_t rc_plan_smem_bytes(int nent) {
+    int n = plan_threads(nent);
+    while (n < nent) n <<= 1;
+    return (size_t)n * (sizeof(unsigned long long) + 5 * sizeof(int)) + 72 * sizeof(int);
 }
 template <int N>
 static size_t segrows_smem() {
@@ -955,7 +998,8 @@ static cudaError_t setup_cols_rc_t() {
 }
 
 cudaError_t segrows_setup(const Plan &P) {
-    cudaError_t e = cudaFuncSetAttribute(k_rc_plan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rc_plan_smem_bytes());
+    cudaError_t e = cudaFuncSetAttribute(k_rc_plan<512, RC_ENTRIES / 512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)rc_plan_smem_bytes(RC_ENTRIES));
     if (e) return e;
     switch (P.npx) {
         case 64: e = setup_segrows_t<64>(); break;
@@ -983,7 +1027,11 @@ size_t rc_max_chunks(int npx, int npy, int nwin) {
 
 void launch_rc_plan(const Plan &P, cudaStream_t s) {
     // one CTA per image unless the host entry wants the chunks listed by row band
-    k_rc_plan<<<P.rc_nbands > 0 ? 1 : 2, PLAN_THREADS, rc_plan_smem_bytes(), s>>>(P);
+    const int ctas = P.rc_nbands > 0 ? 1 : 2, nent = ctas == 1 ? 2 * P.nwin : P.nwin;
+    const size_t sm = rc_plan_smem_bytes(nent);
+    if (nent <= 128) k_rc_plan<128, 1><<<ctas, 128, sm, s>>>(P);
+    else if (nent <= 512) k_rc_plan<512, 1><<<ctas, 512, sm, s>>>(P);
+    else k_rc_plan<512, RC_ENTRIES / 512><<<ctas, 512, sm, s>>>(P);
 }
 
 template <int N>
