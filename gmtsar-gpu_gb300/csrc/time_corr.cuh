@@ -6,7 +6,6 @@
 
 namespace xcg {
 cudaError_t time_setup(const Plan &P);
-size_t time_smem_needed(int nx_corr, int mode);
 void launch_tcorr(const Plan &P, cudaStream_t s);
 void launch_tpeak(const Plan &P, cudaStream_t s);
 }  // namespace xcg

@@ -607,7 +607,7 @@ xcg_status ctx_launch(xcg_ctx *c, Plan P, const int *starts, int nb, cudaStream_
                         }
                         break;
                     case 1:
-                        if (tm) launch_tcorr(Q, ss);
+                        if (tm) { launch_tcorr(Q, ss); c->stats.launches += 2; }     // three kernels
                         else if (rc) launch_cols_rc(Q, ss);
                         else launch_cols(Q, ss);
                         break;

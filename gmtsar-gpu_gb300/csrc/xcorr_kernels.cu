@@ -267,11 +267,14 @@ __global__ void __launch_bounds__(128, (N >= 1024) ? 2 : (N >= 512 ? 3 : 4)) k_r
         };
         if (ir == 0) packed(std::true_type{});
         else packed(std::false_type{});
-        // the precision form transforms the packed rows on the tensor cores
-        if (!P.tc_form) team_fft_reg<N, -1>(v, ex, tw, lane);
-        float2 *zg = P.zrow + ((size_t)w * npy + r) * N;
+        // the precision form transforms the packed rows on the tensor cores;
+        // the time modes need no spectra
+        if (P.corr_mode == 2) {
+            if (!P.tc_form) team_fft_reg<N, -1>(v, ex, tw, lane);
+            float2 *zg = P.zrow + ((size_t)w * npy + r) * N;
 #pragma unroll
-        for (int m = 0; m < PER; m++) zg[lane + T * m] = v[m];
+            for (int m = 0; m < PER; m++) zg[lane + T * m] = v[m];
+        }
         __syncwarp();
     }
     oob = __ballot_sync(0xffffffffu, oob) != 0u;      // any lane of the chunk's warp
