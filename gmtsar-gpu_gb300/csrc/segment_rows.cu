@@ -122,6 +122,7 @@ __device__ __forceinline__ void warp_sort(unsigned long long &k, int &p) {
 template <int NT, int PER>
 __global__ void __launch_bounds__(NT, 1) k_rc_plan(Plan P) {
     const int tid = threadIdx.x;
+    if (P.chain == 1) grid_dep_launch();
     // Two CTAs (no row bands): CTA i plans image i's entries alone, its runs
     // never meeting the other image's, and numbers its chunks from
     // i * nwin * nchunks (the most chunks the master entries can need), so
@@ -335,9 +336,11 @@ __global__ void __launch_bounds__(128, (N >= 1024) ? 2 : (N >= 512 ? 3 : 4)) k_s
                                            (size_t)(blockDim.x / T) * (PADN * sizeof(float2) + (2 * N + RBP) * sizeof(float))) +
                  (size_t)warp * (ACC + RBP);           // [ACC + RBP] first-level sums of the warp's chunk
 
+    if (P.chain == 1) grid_dep_launch();
     for (int i = threadIdx.x; i < TWL; i += blockDim.x) tw[i] = P.tw_row[i];
     if constexpr (HSHIFT)
         for (int i = threadIdx.x; i < TWL; i += blockDim.x) tw[TWL + i] = P.phase[i];
+    grid_dep_wait();                 // the planner's chunks
     __syncthreads();
 
     constexpr int ri = 1 << LG;
@@ -743,6 +746,11 @@ k_cols_rcp(Plan P) {
     // call in single tiles).  Shorter chunks towards the end of a large batch
     // cost more in patch means than the shorter tail gives (1000 windows of
     // 128 x 128: 426 against 420 us).
+    if (P.chain == 1) grid_dep_launch();
+    for (int i = threadIdx.x; i < TWL; i += THR) cp_async8(tw + i, P.tw_col + i);
+    for (int i = threadIdx.x; i < M; i += THR) cp_async8(boxy + i, P.box_y + i);
+    cp_async_commit();               // a group of its own, complete when the first tile's slave rows are
+    grid_dep_wait();                 // the row stage's spectra and sums
     const bool dyn = (P.rc_tile_next != nullptr);
     const int K = max(1, min(NG / 4, ntiles / (2 * (int)gridDim.x)));
     int t, tend;                                // the current chunk [t, tend)
@@ -797,8 +805,6 @@ k_cols_rcp(Plan P) {
 
     stage_slave(t);
     stage_master(t);
-    for (int i = threadIdx.x; i < TWL; i += THR) tw[i] = P.tw_col[i];
-    for (int i = threadIdx.x; i < M; i += THR) boxy[i] = __ldg(P.box_y + i);
 
     int cur_w = -1;
     for (;;) {
@@ -1048,10 +1054,10 @@ static void launch_segrows_t(const Plan &P, cudaStream_t s) {
     const size_t cap = (size_t)sms * per_sm * (P.rc_nbands > 0 ? 2 : 8);
     const int grid = (int)((maxq < cap) ? maxq : cap);
     switch (P.log2ri) {
-        case 0: k_segrows<N, 0><<<grid, 128, segrows_smem<N>(), s>>>(P); break;
-        case 1: k_segrows<N, 1><<<grid, 128, segrows_smem<N>(), s>>>(P); break;
-        case 2: k_segrows<N, 2><<<grid, 128, segrows_smem<N>(), s>>>(P); break;
-        default: k_segrows<N, 3><<<grid, 128, segrows_smem<N>(), s>>>(P); break;
+        case 0: launch_chain(P, k_segrows<N, 0>, dim3(grid), 128, segrows_smem<N>(), s); break;
+        case 1: launch_chain(P, k_segrows<N, 1>, dim3(grid), 128, segrows_smem<N>(), s); break;
+        case 2: launch_chain(P, k_segrows<N, 2>, dim3(grid), 128, segrows_smem<N>(), s); break;
+        default: launch_chain(P, k_segrows<N, 3>, dim3(grid), 128, segrows_smem<N>(), s); break;
     }
 }
 void launch_segrows(const Plan &P, cudaStream_t s) {
@@ -1070,7 +1076,7 @@ static void launch_cols_rc_t(const Plan &P, cudaStream_t s) {
     const int ntiles = ((P.npx / 2) / G::CP) * P.nwin;
     if (P.cols_cfg == 1) {                       // one CTA per tile
         dim3 grid((P.npx / 2) / G::CP, P.nwin);
-        k_cols_rc<M, 128><<<grid, 128, cols_rc_smem<M>(), s>>>(P);
+        k_cols_rc<M, 128><<<grid, 128, cols_rc_smem<M>(), s>>>(P);      // (not a dependent: it does not wait)
         return;
     }
     // persistent: one CTA per resident slot, tiles split into contiguous
@@ -1086,11 +1092,11 @@ static void launch_cols_rc_t(const Plan &P, cudaStream_t s) {
     const bool keep = (P.cols_cfg == 2) != (M <= 256);
     if (keep && G::BLOCKS > 1) {
         const int grid = std::min(ntiles, sms * (G::BLOCKS - 1));
-        k_cols_rcp<M, 128, true><<<grid, 128, cols_rc_smem<M>(), s>>>(P);
+        launch_chain(P, k_cols_rcp<M, 128, true>, dim3(grid), 128, cols_rc_smem<M>(), s);
         return;
     }
     const int grid = std::min(ntiles, sms * G::BLOCKS);
-    k_cols_rcp<M, 128, false><<<grid, 128, cols_rc_smem<M>(), s>>>(P);
+    launch_chain(P, k_cols_rcp<M, 128, false>, dim3(grid), 128, cols_rc_smem<M>(), s);
 }
 void launch_cols_rc(const Plan &P, cudaStream_t s) {
     switch (P.npy) {

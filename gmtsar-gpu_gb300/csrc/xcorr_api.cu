@@ -541,6 +541,14 @@ xcg_status ctx_launch(xcg_ctx *c, Plan P, const int *starts, int nb, cudaStream_
     const int lanes = mode ? 2 * c->nslots : c->nslots;
     const bool fork = nb > 1 && lanes > 1 && c->profiling != 1;
     const bool tl = c->profiling == 2;
+    // the kernels of a batch chained as programmatic dependents (not while
+    // profiling, whose events lie between them, nor into a captured graph,
+    // which keeps plain kernel edges)
+    P.chain = 0;
+    if (rc && c->profiling == 0 && P.cols_cfg != 1) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
+        if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) P.chain = nb == 1 ? 1 : 2;
+    }
     if (tcf) {             // a timeout of an earlier call must not be reported by this one
         const xcg_status rs = tc_reset_status(c, s);
         if (rs != XCG_OK) return rs;
@@ -810,6 +818,7 @@ xcg_status xcg_correlate(xcg_ctx *c, const void *master, int32_t m_nx, int32_t m
             int lo[2], hi[2];
             for (int k = 0; k < 2; k++) rows_of(Q.win0, Q.win0 + Q.nwin, k, lo[k], hi[k]);
             xcg::Plan Qb = Q;
+            Qb.chain = 0;                 // a band's rows wait for its copy, not only for the launch before
             const int nb = std::max(1, std::min(8, Q.nwin / 128));
             Qb.rc_nbands = nb;
             for (int b = 0; b < nb; b++)

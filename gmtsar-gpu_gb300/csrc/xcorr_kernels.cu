@@ -529,8 +529,13 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
         }
         cp_async_commit();
     };
+    if (P.chain == 1) grid_dep_launch();
+    for (int i = threadIdx.x; i < TWL; i += NT) cp_async8(tw + i, P.tw_row + i);
+    cp_async_commit();
+    grid_dep_wait();                                      // the column stage's half spectra
     if (team < nyc / 2) fetch_pair(team);
-    for (int i = threadIdx.x; i < TWL; i += NT) tw[i] = P.tw_row[i];
+    else cp_async_commit();                               // an empty group: the twiddles are the one before it
+    cp_async_wait<1>();
     __syncthreads();
     // The reference's surface is exactly zero when either demeaned patch is
     // (its FFTs of zeros stay zeros); the packed transform here would leave
@@ -844,7 +849,7 @@ __global__ void __launch_bounds__(256, 4) k_subpix(Plan P) {
     __shared__ int holder[NT];
 
     const int w = blockIdx.x, tid = threadIdx.x;
-    if (P.skip && P.skip[w]) return;                  // the refiner answered for this window
+    if (P.chain == 1) grid_dep_launch();
     for (int t = tid; t < NX2 * N2 / 2; t += NT) cp_async16(kys + 2 * t, P.ky + 2 * t);
     cp_async_commit();
     float4 kx[XT][4];                                 // two entries of the row operator's row X per vector
@@ -854,6 +859,11 @@ __global__ void __launch_bounds__(256, 4) k_subpix(Plan P) {
         for (int c = 0; c < 4; c++)
             kx[x][c] = __ldg(reinterpret_cast<const float4 *>(P.kx) + ((tid + x * NT) % NX2) * 4 + c);
     if (tid == 0) { scan[0] = 0; scan[1] = 0x7fffffff; }
+    grid_dep_wait();                                  // the peak stage's neighbourhoods
+    if (P.skip && P.skip[w]) {                        // the refiner answered for this window
+        cp_async_wait<0>();
+        return;
+    }
     int next = 0;
     if (tid < 64) {
         float v = P.md[(size_t)w * 64 + tid];
@@ -1135,12 +1145,12 @@ template <int N>
 static void launch_peak_t(const Plan &P, cudaStream_t s) {
     if constexpr (peak_wide_ok<N>()) {
         if (P.peak_cfg == 2) {
-            k_peak<N, peak_wide_minb<N>(), 512><<<P.nwin, 512, peak_smem<N, 512>(), s>>>(P);
+            launch_chain(P, k_peak<N, peak_wide_minb<N>(), 512>, dim3(P.nwin), 512, peak_smem<N, 512>(), s);
             return;
         }
     }
-    if (P.peak_cfg == 1) k_peak<N, peak_minb<N>(1)><<<P.nwin, 256, peak_smem<N>(), s>>>(P);
-    else k_peak<N, peak_minb<N>(0)><<<P.nwin, 256, peak_smem<N>(), s>>>(P);
+    if (P.peak_cfg == 1) launch_chain(P, k_peak<N, peak_minb<N>(1)>, dim3(P.nwin), 256, peak_smem<N>(), s);
+    else launch_chain(P, k_peak<N, peak_minb<N>(0)>, dim3(P.nwin), 256, peak_smem<N>(), s);
 }
 
 void launch_rows(const Plan &P, cudaStream_t s) {
@@ -1172,10 +1182,10 @@ void launch_peak(const Plan &P, cudaStream_t s) {
 }
 void launch_subpix(const Plan &P, cudaStream_t s) {
     switch (P.ifc) {
-        case 8: k_subpix<8><<<P.nwin, 256, subpix_smem<8>(), s>>>(P); break;
-        case 16: k_subpix<16><<<P.nwin, 256, subpix_smem<16>(), s>>>(P); break;
-        case 32: k_subpix<32><<<P.nwin, 256, subpix_smem<32>(), s>>>(P); break;
-        case 64: k_subpix<64><<<P.nwin, 256, subpix_smem<64>(), s>>>(P); break;
+        case 8: launch_chain(P, k_subpix<8>, dim3(P.nwin), 256, subpix_smem<8>(), s); break;
+        case 16: launch_chain(P, k_subpix<16>, dim3(P.nwin), 256, subpix_smem<16>(), s); break;
+        case 32: launch_chain(P, k_subpix<32>, dim3(P.nwin), 256, subpix_smem<32>(), s); break;
+        case 64: launch_chain(P, k_subpix<64>, dim3(P.nwin), 256, subpix_smem<64>(), s); break;
     }
 }
 
