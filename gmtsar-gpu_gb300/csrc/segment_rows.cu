@@ -297,6 +297,11 @@ __global__ void __launch_bounds__(NT, 1) k_rc_plan(Plan P) {
 
 // ------------------------------------------------------------------ row stage
 
+// twiddle entries k_segrows holds: the transform's, and those with the
+// half-sample shift where factor 2 uses them
+template <int N, int LG>
+__host__ __device__ constexpr int segrows_twiddles() { return (N <= 512 && LG < 2) ? 2 * fft_twiddle_len(N) : fft_twiddle_len(N); }
+
 // One warp per chunk of rows of one image segment; the structure of k_rows
 // (teams of T lanes, the rows t and t + 512 of the chunk through one team,
 // rows in registers in the team layout) with one image instead of a window's
@@ -316,9 +321,10 @@ __global__ void __launch_bounds__(128, (N >= 1024) ? 2 : (N >= 512 ? 3 : 4)) k_s
     constexpr int PER = N / T;
     constexpr int NH = N / 2;
     constexpr bool HSHIFT = (LG == 1) && (N <= 512);
-    constexpr int TWS = (N <= 512) ? 2 * TWL : TWL;
+    constexpr int TWS = segrows_twiddles<N, LG>();
     constexpr int RBP = 32;
     constexpr int GOFF = 32 / TPW;
+    constexpr bool KEEPS = LG >= 2;                     // the row's spectrum is kept for the phases after the first
 
     extern __shared__ float4 smem_raw[];
     float2 *tw = reinterpret_cast<float2 *>(smem_raw);
@@ -332,9 +338,14 @@ __global__ void __launch_bounds__(128, (N >= 1024) ? 2 : (N >= 512 ? 3 : 4)) k_s
     const int rbx = tm & 1;
     float *const rbE = rb + rbx, *const rbO = rb - rbx;
     float *const rbL = (lane & 1) ? rbO : rbE;
-    float *acc = reinterpret_cast<float *>(reinterpret_cast<char *>(tw + TWS) +
-                                           (size_t)(blockDim.x / T) * (PADN * sizeof(float2) + (2 * N + RBP) * sizeof(float))) +
-                 (size_t)warp * (ACC + RBP);           // [ACC + RBP] first-level sums of the warp's chunk
+    char *after = reinterpret_cast<char *>(tw + TWS) +
+                  (size_t)(blockDim.x / T) * (PADN * sizeof(float2) + (2 * N + RBP) * sizeof(float));
+    // KEEPS: each thread's spectrum elements, [PER][32] per warp; the warp's
+    // first-level sums use the same memory once its rows are interpolated
+    float2 *spec = reinterpret_cast<float2 *>(after) + (size_t)warp * PER * 32 + l32;
+    static_assert(!KEEPS || (ACC + RBP) * sizeof(float) <= PER * 32 * sizeof(float2), "sums fit the spectra");
+    float *acc = KEEPS ? reinterpret_cast<float *>(spec - l32)
+                       : reinterpret_cast<float *>(after) + (size_t)warp * (ACC + RBP);   // [ACC + RBP] first-level sums of the warp's chunk
 
     if (P.chain == 1) grid_dep_launch();
     for (int i = threadIdx.x; i < TWL; i += blockDim.x) tw[i] = P.tw_row[i];
@@ -412,14 +423,23 @@ __global__ void __launch_bounds__(128, (N >= 1024) ? 2 : (N >= 512 ? 3 : 4)) k_s
                 const int k = ((lane + T * m) << LG) - N / 2;
                 rowE[k] = amp_of(v[m]);
             }
+            if constexpr (KEEPS) {
+                // ri > 2: one forward transform, its elements kept by the
+                // thread that holds them (registers have no room).  Transforming
+                // the row again for each phase took 150 us where this takes 122
+                // (factor 4, 391 windows of 128 x 64)
+                team_fft_reg<N, -1>(v, ex, tw, lane);
+#pragma unroll
+                for (int m = 0; m < PER; m++) spec[32 * m] = v[m];
+            }
 #pragma unroll 1
             for (int p = 1; p < ri; p++) {
-                if (p > 1) {
-                    uint32_t again[PER];
-                    load_row(r, again);
-                    to_complex(again, v);
+                if constexpr (KEEPS) {
+#pragma unroll
+                    for (int m = 0; m < PER; m++) v[m] = spec[32 * m];
+                } else {
+                    team_fft_reg<N, -1>(v, ex, tw, lane);
                 }
-                team_fft_reg<N, -1>(v, ex, tw, lane);
                 if constexpr (HSHIFT) {
                     team_ifft_half_shift<N>(v, ex, tw + TWL, lane);
                 } else {
@@ -966,14 +986,14 @@ static size_t rc_plan_smem_bytes(int nent) {
     while (n < nent) n <<= 1;
     return (size_t)n * (sizeof(unsigned long long) + 5 * sizeof(int)) + 72 * sizeof(int);
 }
-template <int N>
+template <int N, int LG>
 static size_t segrows_smem() {
     constexpr int T = fft_lanes(N);
     constexpr int ACC = (N >= 1024) ? 1024 : 512;
     const int teams = 128 / T;
-    return fft_twiddle_len(N) * (N <= 512 ? 2 : 1) * sizeof(float2) +
+    return segrows_twiddles<N, LG>() * sizeof(float2) +
            (size_t)teams * (fft_padded_len(N) * sizeof(float2) + (2 * N + 32) * sizeof(float)) +
-           (size_t)(128 / 32) * (ACC + 32) * sizeof(float);
+           (LG >= 2 ? (size_t)128 * (N / T) * sizeof(float2) : (size_t)(128 / 32) * (ACC + 32) * sizeof(float));
 }
 template <int M>
 static size_t cols_rc_smem() {
@@ -985,10 +1005,13 @@ static size_t cols_rc_smem() {
 template <int N>
 static cudaError_t setup_segrows_t() {
     cudaError_t e = cudaSuccess;
-    auto set = [&](auto kern) {
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)segrows_smem<N>());
+    auto set = [&](auto kern, size_t bytes) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     };
-    set(k_segrows<N, 0>); set(k_segrows<N, 1>); set(k_segrows<N, 2>); set(k_segrows<N, 3>);
+    set(k_segrows<N, 0>, segrows_smem<N, 0>());
+    set(k_segrows<N, 1>, segrows_smem<N, 1>());
+    set(k_segrows<N, 2>, segrows_smem<N, 2>());
+    set(k_segrows<N, 3>, segrows_smem<N, 3>());
     return e;
 }
 template <int M>
@@ -1054,10 +1077,10 @@ static void launch_segrows_t(const Plan &P, cudaStream_t s) {
     const size_t cap = (size_t)sms * per_sm * (P.rc_nbands > 0 ? 2 : 8);
     const int grid = (int)((maxq < cap) ? maxq : cap);
     switch (P.log2ri) {
-        case 0: launch_chain(P, k_segrows<N, 0>, dim3(grid), 128, segrows_smem<N>(), s); break;
-        case 1: launch_chain(P, k_segrows<N, 1>, dim3(grid), 128, segrows_smem<N>(), s); break;
-        case 2: launch_chain(P, k_segrows<N, 2>, dim3(grid), 128, segrows_smem<N>(), s); break;
-        default: launch_chain(P, k_segrows<N, 3>, dim3(grid), 128, segrows_smem<N>(), s); break;
+        case 0: launch_chain(P, k_segrows<N, 0>, dim3(grid), 128, segrows_smem<N, 0>(), s); break;
+        case 1: launch_chain(P, k_segrows<N, 1>, dim3(grid), 128, segrows_smem<N, 1>(), s); break;
+        case 2: launch_chain(P, k_segrows<N, 2>, dim3(grid), 128, segrows_smem<N, 2>(), s); break;
+        default: launch_chain(P, k_segrows<N, 3>, dim3(grid), 128, segrows_smem<N, 3>(), s); break;
     }
 }
 void launch_segrows(const Plan &P, cudaStream_t s) {
