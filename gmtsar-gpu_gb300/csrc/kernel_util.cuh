@@ -77,8 +77,8 @@ __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol
 // is the launch: 1000 windows 401 -> 395 us, through host buffers 578 -> 566.
 // (Starting it during the last tile measured the same.)
 template <class Kernel>
-inline void launch_chain(const Plan &P, Kernel kern, dim3 grid, int threads, size_t smem, cudaStream_t s) {
-    if (!P.chain) {
+inline void launch_chain(const Plan &P, Kernel kern, dim3 grid, int threads, size_t smem, cudaStream_t s, int cluster = 1) {
+    if (!P.chain && cluster == 1) {
         kern<<<grid, threads, smem, s>>>(P);
         return;
     }
@@ -87,11 +87,18 @@ inline void launch_chain(const Plan &P, Kernel kern, dim3 grid, int threads, siz
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute at[2];
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    if (P.chain) {
+        at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        at[cfg.numAttrs].val.clusterDim.x = (unsigned)cluster;
+        at[cfg.numAttrs].val.clusterDim.y = 1;
+        at[cfg.numAttrs++].val.clusterDim.z = 1;
+    }
     cudaLaunchKernelEx(&cfg, kern, P);      // an error stays for the caller's cudaGetLastError
 }
 

@@ -16,6 +16,7 @@
 //            as two small dense operators and the argmax of the real part.
 //
 // Every kernel cites the reference stages it replaces.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -476,6 +477,11 @@ __global__ void __launch_bounds__(THR, ColsGeom<M, THR>::BLOCKS) k_cols(Plan P) 
 }
 
 // ---------------------------------------------------------------- k_peak
+// distributed shared memory of a thread-block cluster
+template <class E>
+__device__ __forceinline__ E *on_rank(E *p, int rank) { return cooperative_groups::this_cluster().map_shared_rank(p, rank); }
+__device__ __forceinline__ void cluster_sync() { cooperative_groups::this_cluster().sync(); }
+
 // Replaces the row half of the inverse FFT, d_fillcorrmat_strip/d_Cabs
 // (do_freq_xcorr.cu:26-29,67-84,141-143), h_reduce_strip (conv_ampl_demean.cu:642-675),
 // the per-window host loop of d_do_freq_corr_strip (do_freq_xcorr.cu:150-195),
@@ -484,7 +490,10 @@ __global__ void __launch_bounds__(THR, ColsGeom<M, THR>::BLOCKS) k_cols(Plan P) 
 // row pairs of the largest surface (nyc = 512: windows of 512 rows)
 constexpr int PEAK_MAX_ROW_PAIRS = 256;
 
-template <int N, int MINB, int NT = 256>
+// CL: CTAs per window, a cluster that shares the window's row pairs and the time
+// correlation's rows; rank 0 forms the record.  One CTA (CL 1) takes 19 us for
+// a window of 128 x 128 however few windows there are, most of it latency.
+template <int N, int MINB, int NT = 256, int CL = 1>
 __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
     constexpr int T = fft_lanes(N);
     constexpr int PADN = fft_padded_len(N);
@@ -505,14 +514,20 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
     float *rowh = rowf + PEAK_MAX_ROW_PAIRS;
     __shared__ int scan[2];                               // threads that hold the maximum, its position
     __shared__ unsigned short holder[NT];
+    // per rank of the cluster: largest value, its position, the time sums (kept by rank 0)
+    __shared__ unsigned cl_max[CL];
+    __shared__ int cl_pos[CL];
+    __shared__ long long cl_sum[CL][3];
 
-    const int w = blockIdx.x;
+    const int w = blockIdx.x / CL, rank = blockIdx.x % CL;
     const int warp = threadIdx.x >> 5, l32 = threadIdx.x & 31;
     const int lane = l32 % T;
     const int team = warp * (32 / T) + l32 / T;
+    const int pr0 = team + teams * rank;                  // this team's row pairs: pr0, pr0 + teams CL, ...
     float2 *ex = fb + team * PADN;
     const int M = P.npy, nxc = P.nxc, nyc = P.nyc;
     const float scale = 1.0f / ((float)N * (float)M);
+    if constexpr (CL > 1) cooperative_groups::this_cluster().barrier_arrive();   // every CTA of the cluster has started ...
 
     // A row pair's half spectra are copied into the team's exchange buffer
     // (free between transforms) while the previous pair's values are still
@@ -533,10 +548,11 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
     for (int i = threadIdx.x; i < TWL; i += NT) cp_async8(tw + i, P.tw_row + i);
     cp_async_commit();
     grid_dep_wait();                                      // the column stage's half spectra
-    if (team < nyc / 2) fetch_pair(team);
+    if (pr0 < nyc / 2) fetch_pair(pr0);
     else cp_async_commit();                               // an empty group: the twiddles are the one before it
     cp_async_wait<1>();
     __syncthreads();
+    if constexpr (CL > 1) cooperative_groups::this_cluster().barrier_wait();     // ... before any writes into another
     // The reference's surface is exactly zero when either demeaned patch is
     // (its FFTs of zeros stay zeros); the packed transform here would leave
     // rounding residue of the other patch, so that case is set explicitly.
@@ -586,7 +602,7 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
     bool synced = false;                                  // bc written by warp 0, seen by all
     float lmax = 0.f;                                     // the largest value of this thread, if positive
     float *surf = P.surf + (size_t)w * nyc * nxc;
-    for (int pr = team; pr < nyc / 2; pr += teams) {      // the same trips for every team of a warp
+    for (int pr = pr0; pr < nyc / 2; pr += teams * CL) {  // the same trips for every team of a warp
         const int y1 = 2 * pr, y2 = y1 + 1;
         // two real rows in one complex inverse FFT: S = Q1 + i Q2, Hermitian-extended
         cp_async_wait<0>();
@@ -602,7 +618,7 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
         }
         __syncwarp();
         team_fft_reg<N, +1>(v, ex, tw, lane);
-        if (pr + teams < nyc / 2) fetch_pair(pr + teams);
+        if (pr + teams * CL < nyc / 2) fetch_pair(pr + teams * CL);
         if (!synced) {
             __syncthreads();
             keep = (float)bc[2];
@@ -631,7 +647,10 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
             fpart += __shfl_xor_sync(0xffffffffu, fpart, o);
             hpart += __shfl_xor_sync(0xffffffffu, hpart, o);
         }
-        if (lane == 0) { rowf[pr] = fpart; rowh[pr] = hpart; }
+        if (lane == 0) {
+            if constexpr (CL == 1) { rowf[pr] = fpart; rowh[pr] = hpart; }
+            else { on_rank(rowf, 0)[pr] = fpart; on_rank(rowh, 0)[pr] = hpart; }
+        }
     }
     if (!synced) __syncthreads();                         // a warp without row pairs
     // The argmax in two phases: the largest value first, then its position
@@ -650,10 +669,16 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
         unsigned m = 0;
 #pragma unroll
         for (int i = 0; i < NW; i++) m = max(m, (unsigned)rk[i]);
+        if constexpr (CL > 1) {
+            if (threadIdx.x < CL) on_rank(cl_max, threadIdx.x)[rank] = m;
+            cluster_sync();                               // also: every rank's surface rows and row sums are written
+#pragma unroll
+            for (int i = 0; i < CL; i++) m = max(m, cl_max[i]);
+        }
         vmax = __uint_as_float(m);
     }
     if (vmax > 0.f && lmax == vmax) holder[atomicAdd(&scan[0], 1)] = (unsigned short)threadIdx.x;
-    if (warp == NW - 1) {
+    if (warp == NW - 1 && rank == 0) {
         double hs = 0.0, fs = 0.0;
         for (int i = l32; i < nyc / 2; i += 32) { hs += (double)rowh[i]; fs += (double)rowf[i]; }
         hs = warp_sum_f64(hs);
@@ -664,12 +689,12 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
     {
         // a holder's elements: both rows of its team's row pairs, its lane's columns
         constexpr int CPL = PER / 2;                      // surface columns per lane
-        const int per = 2 * CPL * ((nyc / 2 + teams - 1) / teams);
+        const int per = 2 * CPL * ((nyc / 2 + teams * CL - 1) / (teams * CL));
         const int nh = scan[0];
         for (int i = threadIdx.x; i < nh * per; i += NT) {
             const int h = i / per, j = i - h * per;
             const int th = holder[h], hl = (th & 31) % T, ht = (th >> 5) * (32 / T) + (th & 31) / T;
-            const int y = 2 * (ht + (j / (2 * CPL)) * teams) + (j & 1);
+            const int y = 2 * (ht + teams * (rank + CL * (j / (2 * CPL)))) + (j & 1);
             const int x = hl + T * ((j >> 1) % CPL + PER / 4) - nxc / 2;
             if (y < nyc) {
                 const unsigned e = (unsigned)(y * nxc + x);
@@ -678,7 +703,14 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
         }
     }
     __syncthreads();
-    const unsigned pos = (vmax > 0.f) ? (unsigned)scan[1] : 0u;
+    int first = scan[1];
+    if constexpr (CL > 1) {
+        if (threadIdx.x < CL) on_rank(cl_pos, threadIdx.x)[rank] = first;
+        cluster_sync();
+#pragma unroll
+        for (int i = 0; i < CL; i++) first = min(first, cl_pos[i]);
+    }
+    const unsigned pos = (vmax > 0.f) ? (unsigned)first : 0u;
     const unsigned pk = argmax_order(pos);
     const int ip = (int)(pk / (unsigned)nxc), jp = (int)(pk % (unsigned)nxc);
     const double cmax = (double)vmax;
@@ -717,9 +749,10 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
         float *st = reinterpret_cast<float *>(fb);
         const int ash = (int)((unsigned)jp & 3u);
         const float *a1q = a1 - ash;
+        const int rbeg = P.ny_corr / CL * rank, rend = P.ny_corr / CL * (rank + 1);   // this rank's rows
         auto stage = [&](int r0, int half) {
             float *sa = st + half * RR * (SA + NXC), *sb = sa + RR * SA;
-            const int n = min(RR, P.ny_corr - r0);
+            const int n = min(RR, rend - r0);
             for (int i = threadIdx.x; i < n * (SA / 4); i += NT) {
                 const int r = i / (SA / 4), c = 4 * (i - r * (SA / 4));
                 cp_async16(sa + r * SA + c, a1q + (size_t)(r0 + r) * N + c);
@@ -730,9 +763,9 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
             }
             cp_async_commit();
         };
-        stage(0, 0);
-        for (int r0 = 0, half = 0; r0 < P.ny_corr; r0 += RR, half ^= 1) {
-            if (r0 + RR < P.ny_corr) {
+        stage(rbeg, 0);
+        for (int r0 = rbeg, half = 0; r0 < rend; r0 += RR, half ^= 1) {
+            if (r0 + RR < rend) {
                 stage(r0 + RR, half ^ 1);
                 cp_async_wait<1>();
             } else {
@@ -740,7 +773,7 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
             }
             __syncthreads();
             const float *sa = st + half * RR * (SA + NXC) + ash, *sb = st + half * RR * (SA + NXC) + RR * SA;
-            const int n = min(RR, P.ny_corr - r0) * NXC;
+            const int n = min(RR, rend - r0) * NXC;
 #pragma unroll 4
             for (int i = threadIdx.x; i < n; i += NT) {
                 const int r = i / NXC, cc = i - r * NXC;
@@ -753,9 +786,22 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
     sn = warp_sum_i64(sn); s1 = warp_sum_i64(s1); s2 = warp_sum_i64(s2);
     if (l32 == 0) { ri64[warp] = sn; ri64[NW + warp] = s1; ri64[2 * NW + warp] = s2; }
     __syncthreads();
+    if constexpr (CL > 1) {
+        if (threadIdx.x < 3) {
+            long long t = 0;
+            for (int i = 0; i < NW; i++) t += ri64[threadIdx.x * NW + i];
+            on_rank(&cl_sum[0][0], 0)[rank * 3 + threadIdx.x] = t;
+        }
+        cluster_sync();
+        if (rank != 0) return;            // nothing of this CTA's is read any more
+    }
     if (threadIdx.x == 0) {
         long long tn = 0, t1 = 0, t2 = 0;
-        for (int i = 0; i < NW; i++) { tn += ri64[i]; t1 += ri64[NW + i]; t2 += ri64[2 * NW + i]; }
+        if constexpr (CL == 1) {
+            for (int i = 0; i < NW; i++) { tn += ri64[i]; t1 += ri64[NW + i]; t2 += ri64[2 * NW + i]; }
+        } else {
+            for (int i = 0; i < CL; i++) { tn += cl_sum[i][0]; t1 += cl_sum[i][1]; t2 += cl_sum[i][2]; }
+        }
         const double gd = sqrt(1.0 * (double)t1 * (double)t2);
         const double gamma = (gd == 0.0) ? 0.0 : 100.0 * fabs((double)tn / gd);
         const double msc = cmax / gamma;
@@ -1038,6 +1084,12 @@ static size_t cols_smem(int) {
     using G = ColsGeom<M, THR>;
     return G::TWL * sizeof(float2) + (size_t)2 * G::CP * G::CS * sizeof(float2) + 2 * sizeof(double);
 }
+// A cluster of four CTAs per window while all of them fit the GPU at once (four
+// per SM) and each rank's teams have a row pair: with their launches, 20
+// windows of 128 x 128 22.2 -> 14.9 us, 140 of them 24.6 -> 22.6, 20 of 256 x
+// 256 57 -> 26.5.  More windows hide each other's latency (200: the same), and
+// ranks without rows only wait (100 windows of 64 x 64: 14.3 -> 18.4 us).
+constexpr int PEAK_CL = 4, PEAK_CL_WINDOWS = 152;
 // resident k_peak CTAs per SM for configuration cfg
 template <int N>
 constexpr int peak_minb(int cfg) { return (N <= 256) ? (cfg == 1 ? 3 : 4) : (N <= 512 ? (cfg == 1 ? 2 : 3) : 1); }
@@ -1084,6 +1136,9 @@ template <int N>
 static cudaError_t setup_peak() {
     cudaError_t e = cudaFuncSetAttribute(k_peak<N, peak_minb<N>(0)>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)peak_smem<N>());
+    if (!e)
+        e = cudaFuncSetAttribute(k_peak<N, peak_minb<N>(0), 256, PEAK_CL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)peak_smem<N>());
     if (!e && peak_minb<N>(1) != peak_minb<N>(0))
         e = cudaFuncSetAttribute(k_peak<N, peak_minb<N>(1)>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)peak_smem<N>());
@@ -1143,6 +1198,10 @@ static void launch_cols_t(const Plan &P, cudaStream_t s) {
 }
 template <int N>
 static void launch_peak_t(const Plan &P, cudaStream_t s) {
+    if (P.nwin <= PEAK_CL_WINDOWS && P.nyc / 2 >= PEAK_CL * (256 / fft_lanes(N)) && P.peak_cfg == 0) {
+        launch_chain(P, k_peak<N, peak_minb<N>(0), 256, PEAK_CL>, dim3(P.nwin * PEAK_CL), 256, peak_smem<N>(), s, PEAK_CL);
+        return;
+    }
     if constexpr (peak_wide_ok<N>()) {
         if (P.peak_cfg == 2) {
             launch_chain(P, k_peak<N, peak_wide_minb<N>(), 512>, dim3(P.nwin), 512, peak_smem<N, 512>(), s);
