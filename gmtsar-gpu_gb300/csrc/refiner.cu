@@ -7,9 +7,11 @@
 //
 // Network (valid 3x3 convolutions, GELU): 9x9 -> 32@7x7 -> 32@5x5 -> 32@3x3
 // -> dense 64 -> dense 3.  37,507 parameters, FP32 master copy.
-//   training:  k_ref_fwd (FP32, keeps activations and GELU derivatives) ->
-//              k_ref_bwd (activation gradients) -> k_ref_wgrad (partial
-//              parameter gradients) -> k_ref_reduce -> k_ref_adam
+//   training:  k_ref_fwd (the convolutions, FP32, keeps activations and GELU
+//              derivatives) -> k_ref_dense (the dense layers forward, the
+//              loss, and back) -> k_ref_bwd (the convolutions back) ->
+//              k_ref_wgrad (partial parameter gradients) -> k_ref_reduce ->
+//              k_ref_adam
 //   inference: k_ref_infer, BF16 weights and activations on the tensor cores
 //              (mma.sync m16n8k16, FP32 accumulation), conv+GELU fused with
 //              the activations channel-last in shared memory, one CTA per
@@ -34,373 +36,449 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
 }
 
 // ---------------------------------------------------------------- training kernels
-// FP32 multiply-adds bound all three: 1.04 M per sample in all, 0.11 ms per
-// 4096 samples at the measured FP32 rate.  Each keeps its operands in shared
-// memory, reads them as 16-byte vectors that most lanes of a warp share, and
-// holds a register tile of outputs, so that a shared-memory read feeds 6 to 16
-// multiply-adds.  One CTA per SM; a CTA takes a contiguous range of samples.
-// A gradient of 4096 samples: 4.34 -> 0.44 ms; one warp per sample with scalar
-// reads, and the parameter gradients gathered with a lane stride of a whole
-// 21.8 KB record (2.7 ms of the 4.3), against 0.16 + 0.12 + 0.09 + 0.01 ms.
-// What bounds them now: barriers between the layers (forward, backward),
-// issue (parameter gradients).
+// FP32 multiply-adds bound them: 1.04 M per sample in all, 0.11 ms per 4096
+// samples at the measured FP32 rate.  In the convolutions a thread holds all
+// outputs of one channel of one sample, so a shared-memory read (a row that the
+// whole warp shares, or one weight per lane) feeds 4 to 10 of them; the layers
+// run as roles of different warps on successive groups of four samples, one
+// barrier per group, every scheduler with one warp of each role.  One CTA per SM
+// takes a contiguous range of samples.  A gradient of 4096 samples with its host
+// copies: 338 us (layer after layer on one group at a time, a barrier between
+// layers: 437; a thread per output in one kernel each way: 4340).
 
 // Activation rows are padded to 8 floats (4 for the 3-wide rows), channels to
-// strides whose 16-byte reads by consecutive lanes hit distinct banks, samples
-// to strides that are 8 modulo 32 words.
-constexpr int TR_S = 8;                        // samples of a group in shared memory
+// strides whose 16-byte accesses by consecutive lanes hit distinct banks.
+constexpr int TR_S = 4;                        // samples of a group
 constexpr int X0_S = 108, X0_R = 12;           // input: sample stride, row stride
-constexpr int A1_SS = 1928, A2_SS = 1416, A3_SS = 292;     // sample strides in the forward kernel
-constexpr int DY2_SS = 1288, DY3_SS = 392;                 // in the backward kernel
+constexpr int A3_SS = 292;                     // dense input: sample stride in shared memory
 
 __device__ __forceinline__ void ld4(float *d, const float *s) {
     const float4 v = *reinterpret_cast<const float4 *>(s);
     d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
 }
-// gelu_f and, when G, gelu_g from one erff
+// GELU and, when G, its derivative from one erff
 template <bool G>
 __device__ __forceinline__ float gelu_both(float x, float &grad) {
     const float e = erff(x * 0.70710678118654752f);
     if (G) grad = 0.5f * (1.0f + e) + x * 0.39894228040143268f * expf(-0.5f * x * x);
     return 0.5f * x * (1.0f + e);
 }
+// a shared array (size and addresses multiples of 16 bytes) to global memory, by one thread
+__device__ __forceinline__ void bulk_out(float *gmem, const float *smem, int bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\n" ::"l"(gmem),
+                 "r"((unsigned)__cvta_generic_to_shared(smem)), "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;\n" ::: "memory"); }
+// all but the N newest groups have read their shared memory / are complete
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;\n" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory"); }
+__device__ __forceinline__ void fence_bulk() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 
-// One output row of a valid 3x3 convolution for channels c, c + 1: WO outputs
-// each, 32 input channels, the input rows (WO + 2 wide, stride 8) at `in`,
-// weights [k][tap][c].  The sum runs over the input channels, then the taps.
+// A valid 3x3 convolution of one sample for output channel c: WO x WO sums, 32
+// input channels in_cs apart at `in` (rows of 8), weights [k][tap][c].  Each
+// sum runs over the input channels, then the taps.
 template <int WO>
-__device__ __forceinline__ void conv_row(float (&y)[2][WO], const float *in, int in_cs, const float *W, int c) {
-#pragma unroll 2
+__device__ __forceinline__ void conv_all(float (&y)[WO][WO], const float *in, int in_cs, const float *W, int c) {
+#pragma unroll 1
     for (int k = 0; k < 32; k++) {
+        float w[9];
 #pragma unroll
-        for (int di = 0; di < 3; di++) {
+        for (int d = 0; d < 9; d++) w[d] = W[(k * 9 + d) * 32 + c];
+#pragma unroll
+        for (int r = 0; r < WO + 2; r++) {
             float x[8];
-            ld4(x, in + k * in_cs + di * 8);
-            ld4(x + 4, in + k * in_cs + di * 8 + 4);
+            ld4(x, in + k * in_cs + r * 8);
+            ld4(x + 4, in + k * in_cs + r * 8 + 4);
 #pragma unroll
-            for (int dj = 0; dj < 3; dj++) {
-                const float2 w = *reinterpret_cast<const float2 *>(W + (k * 9 + di * 3 + dj) * 32 + c);
+            for (int di = 0; di < 3; di++) {
+                if (r - di < 0 || r - di >= WO) continue;
 #pragma unroll
-                for (int j = 0; j < WO; j++) {
-                    y[0][j] = fmaf(w.x, x[j + dj], y[0][j]);
-                    y[1][j] = fmaf(w.y, x[j + dj], y[1][j]);
-                }
+                for (int dj = 0; dj < 3; dj++)
+#pragma unroll
+                    for (int j = 0; j < WO; j++) y[r - di][j] = fmaf(w[di * 3 + dj], x[j + dj], y[r - di][j]);
             }
         }
     }
 }
 
-// Forward pass: a task is (sample, output row, two channels); the warps of
-// one output row share their scheduler slots evenly (four warps per row).
-// TRAIN: the activations and the GELU derivatives go to the sample's record.
-constexpr int FWD_THREADS = 640;
+// The convolutions' forward pass.  Warps 0-3: conv2, 4-7: conv3, 8-11: conv1,
+// a warp per sample, a lane per channel; in one step conv1 works on group t,
+// conv2 on t - 1, conv3 on t - 2.  TRAIN: the activations and the GELU
+// derivatives go to the sample's record, else only conv3's activations.
+constexpr int FWD_THREADS = 384;
 template <bool TRAIN>
 __global__ void __launch_bounds__(FWD_THREADS, 1) k_ref_fwd(RefPlan R, const float *__restrict__ feat, int n) {
     extern __shared__ float4 smem_v[];
     float *W2 = reinterpret_cast<float *>(smem_v);     // [k*9 + tap][c]
     float *W3 = W2 + 9216;
-    float *x0 = W3 + 9216, *a1 = x0 + TR_S * X0_S, *a2 = a1 + TR_S * A1_SS, *a3 = a2 + TR_S * A2_SS,
-          *g1 = a3 + TR_S * A3_SS;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float *a1 = W3 + 9216;                             // [2][TR_S][A1_LEN] by the group's parity
+    float *a2 = a1 + 2 * TR_S * A1_LEN;                // [2][TR_S][A2_LEN]
+    float *x0 = a2 + 2 * TR_S * A2_LEN;                // [TR_S][X0_S]
+    const int tid = threadIdx.x, c = tid & 31, warp = tid >> 5, s = warp & 3, role = warp >> 2;
+    const int per = (n + gridDim.x - 1) / gridDim.x;
+    const int s_beg = blockIdx.x * per, s_end = min(n, s_beg + per);
+    if (s_beg >= s_end) return;
     for (int i = tid; i < 9216 / 4; i += FWD_THREADS) {
         reinterpret_cast<float4 *>(W2)[i] = reinterpret_cast<const float4 *>(R.w2t)[i];
         reinterpret_cast<float4 *>(W3)[i] = reinterpret_cast<const float4 *>(R.w3t)[i];
     }
     const float *P = R.theta;
-    const int per = (n + gridDim.x - 1) / gridDim.x;
-    const int s_end = min(n, (int)(blockIdx.x + 1) * per);
-    const int c = 2 * (lane & 15);                     // this task's channels c, c + 1
-    const int q = warp & 3;                            // with the lane's half: the task's sample
-    const int s = 2 * q + (lane >> 4);
-    for (int s0 = blockIdx.x * per; s0 < s_end; s0 += TR_S) {
-        const int m = min(TR_S, s_end - s0);
-        const bool have = s < m;
-        float *rec = R.act + (size_t)(s0 + (have ? s : 0)) * REF_ACT;
-        for (int i = tid; i < m * 81; i += FWD_THREADS) {
-            const int ss = i / 81, e = i - ss * 81;
-            x0[ss * X0_S + (e / 9) * X0_R + e % 9] = feat[(size_t)s0 * 81 + i];
-        }
-        __syncthreads();
-        if (have)
-            for (int row = warp >> 2; row < 7; row += FWD_THREADS / 128) {     // conv1
-                float y[2][7], w[2][9];
+    const int groups = (s_end - s_beg + TR_S - 1) / TR_S;
+    float w1[9], bias = P[(role == 0 ? RP_B2 : role == 1 ? RP_B3 : RP_B1) + c];
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const float b = P[RP_B1 + c + h];
+    for (int d = 0; d < 9; d++) w1[d] = __ldg(P + RP_W1 + c * 9 + d);
+    float nx[3] = {0.f, 0.f, 0.f};                     // conv1: the next group's input, 81 values over the lanes
+    auto fetch = [&](int g) {
+        const int at = s_beg + g * TR_S + s;
 #pragma unroll
-                    for (int j = 0; j < 7; j++) y[h][j] = b;
+        for (int q = 0; q < 3; q++) nx[q] = (at < s_end && c + 32 * q < 81) ? feat[(size_t)at * 81 + c + 32 * q] : 0.f;
+    };
+    if (role == 2) fetch(0);
+    __syncthreads();
+    for (int t = 0; t < groups + 2; t++) {
+        const int g = t - (role == 2 ? 0 : role == 0 ? 1 : 2);      // this role's group
+        const int at = s_beg + g * TR_S + s;
+        const bool have = g >= 0 && g < groups && at < s_end;
+        float *rec = R.act + (size_t)(have ? at : s_beg) * REF_ACT;
+        const int buf = g & 1;
+        if (role == 2) {                               // conv1
+            float *xs = x0 + s * X0_S;
 #pragma unroll
-                    for (int d = 0; d < 9; d++) w[h][d] = __ldg(P + RP_W1 + (c + h) * 9 + d);
-                }
+            for (int q = 0; q < 3; q++) {
+                const int e = c + 32 * q;
+                if (e < 81) xs[(e / 9) * X0_R + e % 9] = nx[q];
+            }
+            __syncwarp();
+            fetch(g + 1);
+            if (have) {
+                float *out = a1 + (buf * TR_S + s) * A1_LEN + c * A1_CS;
+#pragma unroll 1
+                for (int row = 0; row < 7; row++) {
+                    float y[7], a[8], gd[8];
 #pragma unroll
-                for (int di = 0; di < 3; di++) {
-                    float x[12];
-                    const float *xr = x0 + s * X0_S + (row + di) * X0_R;
-                    ld4(x, xr); ld4(x + 4, xr + 4); ld4(x + 8, xr + 8);
+                    for (int j = 0; j < 7; j++) y[j] = bias;
 #pragma unroll
-                    for (int dj = 0; dj < 3; dj++)
+                    for (int di = 0; di < 3; di++) {
+                        float x[12];
+                        const float *xr = xs + (row + di) * X0_R;
+                        ld4(x, xr); ld4(x + 4, xr + 4); ld4(x + 8, xr + 8);
 #pragma unroll
-                        for (int j = 0; j < 7; j++) {
-                            y[0][j] = fmaf(w[0][di * 3 + dj], x[j + dj], y[0][j]);
-                            y[1][j] = fmaf(w[1][di * 3 + dj], x[j + dj], y[1][j]);
-                        }
-                }
+                        for (int dj = 0; dj < 3; dj++)
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    float a[8], g[8];
-                    a[7] = g[7] = 0.f;
+                            for (int j = 0; j < 7; j++) y[j] = fmaf(w1[di * 3 + dj], x[j + dj], y[j]);
+                    }
+                    a[7] = gd[7] = 0.f;
 #pragma unroll
-                    for (int j = 0; j < 7; j++) a[j] = gelu_both<TRAIN>(y[h][j], g[j]);
+                    for (int j = 0; j < 7; j++) a[j] = gelu_both<TRAIN>(y[j], gd[j]);
 #pragma unroll
                     for (int v = 0; v < 2; v++) {
-                        const float4 av = make_float4(a[4 * v], a[4 * v + 1], a[4 * v + 2], a[4 * v + 3]);
-                        *reinterpret_cast<float4 *>(a1 + s * A1_SS + (c + h) * A1_CS + row * 8 + 4 * v) = av;
-                        if (TRAIN) {
-                            *reinterpret_cast<float4 *>(rec + ACT_A1 + (c + h) * A1_CS + row * 8 + 4 * v) = av;
-                            *reinterpret_cast<float4 *>(rec + ACT_D1 + (c + h) * 56 + row * 8 + 4 * v) =
-                                make_float4(g[4 * v], g[4 * v + 1], g[4 * v + 2], g[4 * v + 3]);
-                        }
+                        *reinterpret_cast<float4 *>(out + row * 8 + 4 * v) = make_float4(a[4 * v], a[4 * v + 1], a[4 * v + 2], a[4 * v + 3]);
+                        if (TRAIN)
+                            *reinterpret_cast<float4 *>(rec + ACT_D1 + c * 56 + row * 8 + 4 * v) =
+                                make_float4(gd[4 * v], gd[4 * v + 1], gd[4 * v + 2], gd[4 * v + 3]);
                     }
                 }
             }
-        __syncthreads();
-        if (have && warp < 20) {                       // conv2: row warp / 4
-            const int row = warp >> 2;
-            float y[2][5];
+            __syncwarp();
+        } else if (role == 0) {                        // conv2
+            if (have) {
+                float y[5][5];
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const float b = P[RP_B2 + c + h];
+                for (int i = 0; i < 5; i++)
 #pragma unroll
-                for (int j = 0; j < 5; j++) y[h][j] = b;
-            }
-            conv_row<5>(y, a1 + s * A1_SS + row * 8, A1_CS, W2, c);
+                    for (int j = 0; j < 5; j++) y[i][j] = bias;
+                conv_all<5>(y, a1 + (buf * TR_S + s) * A1_LEN, A1_CS, W2, c);
+                float *out = a2 + (buf * TR_S + s) * A2_LEN + c * A2_CS;
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                float a[8], g[8];
+                for (int i = 0; i < 5; i++) {
+                    float a[8], gd[8];
 #pragma unroll
-                for (int j = 5; j < 8; j++) a[j] = g[j] = 0.f;
+                    for (int j = 5; j < 8; j++) a[j] = gd[j] = 0.f;
 #pragma unroll
-                for (int j = 0; j < 5; j++) a[j] = gelu_both<TRAIN>(y[h][j], g[j]);
+                    for (int j = 0; j < 5; j++) a[j] = gelu_both<TRAIN>(y[i][j], gd[j]);
 #pragma unroll
-                for (int v = 0; v < 2; v++) {
-                    const float4 av = make_float4(a[4 * v], a[4 * v + 1], a[4 * v + 2], a[4 * v + 3]);
-                    *reinterpret_cast<float4 *>(a2 + s * A2_SS + (c + h) * A2_CS + row * 8 + 4 * v) = av;
-                    if (TRAIN) {
-                        *reinterpret_cast<float4 *>(rec + ACT_A2 + (c + h) * A2_CS + row * 8 + 4 * v) = av;
-                        *reinterpret_cast<float4 *>(rec + ACT_D2 + (c + h) * 40 + row * 8 + 4 * v) =
-                            make_float4(g[4 * v], g[4 * v + 1], g[4 * v + 2], g[4 * v + 3]);
+                    for (int v = 0; v < 2; v++) {
+                        *reinterpret_cast<float4 *>(out + i * 8 + 4 * v) = make_float4(a[4 * v], a[4 * v + 1], a[4 * v + 2], a[4 * v + 3]);
+                        if (TRAIN)
+                            *reinterpret_cast<float4 *>(rec + ACT_D2 + c * 40 + i * 8 + 4 * v) =
+                                make_float4(gd[4 * v], gd[4 * v + 1], gd[4 * v + 2], gd[4 * v + 3]);
                     }
                 }
             }
-        }
-        __syncthreads();
-        if (have && warp < 12) {                       // conv3: row warp / 4
-            const int row = warp >> 2;
-            float y[2][3];
+        } else if (have) {                             // conv3
+            float y[3][3];
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const float b = P[RP_B3 + c + h];
+            for (int i = 0; i < 3; i++)
 #pragma unroll
-                for (int j = 0; j < 3; j++) y[h][j] = b;
-            }
-            conv_row<3>(y, a2 + s * A2_SS + row * 8, A2_CS, W3, c);
+                for (int j = 0; j < 3; j++) y[i][j] = bias;
+            conv_all<3>(y, a2 + (buf * TR_S + s) * A2_LEN, A2_CS, W3, c);
 #pragma unroll
-            for (int h = 0; h < 2; h++)
+            for (int i = 0; i < 3; i++)
 #pragma unroll
                 for (int j = 0; j < 3; j++) {
-                    float g;
-                    const float a = gelu_both<TRAIN>(y[h][j], g);
-                    const int e = (c + h) * 9 + row * 3 + j;
-                    a3[s * A3_SS + e] = a;
-                    if (TRAIN) { rec[ACT_A3 + e] = a; rec[ACT_D3 + e] = g; }
+                    float gd;
+                    const float a = gelu_both<TRAIN>(y[i][j], gd);
+                    rec[ACT_A3 + c * 9 + i * 3 + j] = a;
+                    if (TRAIN) rec[ACT_D3 + c * 9 + i * 3 + j] = gd;
                 }
         }
+        // the activations written in this step go out while the next step reads
+        // them; a buffer is written again two steps later
+        if (TRAIN) {
+            if (c == 0 && role != 1) bulk_wait_read<0>();      // this warp's copy of the step before
+            fence_bulk();
+        }
         __syncthreads();
-        if (tid < 256) {                               // dense 288 -> 64: output o of samples 2 sp, 2 sp + 1
-            const int o = tid & 63, sp = tid >> 6;
-            float z0 = P[RP_C1 + o], z1 = z0;
-            const float *p0 = a3 + (2 * sp) * A3_SS, *p1 = p0 + A3_SS;
+        if (TRAIN && c == 0 && have) {
+            if (role == 2) bulk_out(rec + ACT_A1, a1 + (buf * TR_S + s) * A1_LEN, A1_LEN * 4);
+            if (role == 0) bulk_out(rec + ACT_A2, a2 + (buf * TR_S + s) * A2_LEN, A2_LEN * 4);
+            bulk_commit();
+        }
+    }
+    if (TRAIN && c == 0) bulk_wait_all();
+}
+
+// The dense layers of 32 samples per CTA, forward (288 -> 64 -> 3), and in
+// training the loss and the gradients back to conv3's pre-activations.  A
+// thread's forward tile is 4 outputs x 2 samples (each sum over the inputs in
+// order), its backward tile 9 inputs x 4 samples.
+constexpr int DN_S = 32, DN_THREADS = 256, F1_S = 68, Z_S = 68;    // samples, threads, padded row strides
+template <bool TRAIN>
+__global__ void __launch_bounds__(DN_THREADS, 1) k_ref_dense(RefPlan R, const float *__restrict__ target, int n) {
+    extern __shared__ float4 smem_v[];
+    float *F1 = reinterpret_cast<float *>(smem_v);     // [288][F1_S]: (input, output)
+    float *a3 = F1 + 288 * F1_S;                       // [DN_S][A3_SS]
+    float *g1 = a3 + DN_S * A3_SS;                     // [DN_S][Z_S] outputs of the first layer, then their gradients
+    float *dg = g1 + DN_S * Z_S;                       // [DN_S][Z_S] GELU derivatives
+    float *F2 = dg + DN_S * Z_S;                       // [3][64]
+    float *dout = F2 + 192;                            // [DN_S][4]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int s0 = blockIdx.x * DN_S, m = min(DN_S, n - s0);
+    const float *P = R.theta;
+    for (int i = tid; i < 288 * 16; i += DN_THREADS) cp_async16(F1 + (i >> 4) * F1_S + 4 * (i & 15), R.f1t + 4 * i);
+    for (int i = tid; i < DN_S * 72; i += DN_THREADS) {
+        const int ss = i / 72, e = i - 72 * ss;
+        if (ss < m) cp_async16(a3 + ss * A3_SS + 4 * e, R.act + (size_t)(s0 + ss) * REF_ACT + ACT_A3 + 4 * e);
+        else *reinterpret_cast<float4 *>(a3 + ss * A3_SS + 4 * e) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+    if (tid < 192) F2[tid] = P[RP_F2 + tid];
+    __syncthreads();
+    {
+        const int o = 4 * (tid & 15), sp = 2 * (tid >> 4);
+        float z[2][4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) z[0][k] = z[1][k] = P[RP_C1 + o + k];
+        const float *p0 = a3 + sp * A3_SS, *p1 = p0 + A3_SS;
 #pragma unroll 4
-            for (int h = 0; h < 288; h += 4) {
-                float w[4], u0[4], u1[4];
+        for (int h = 0; h < 288; h += 4) {
+            float u0[4], u1[4];
+            ld4(u0, p0 + h);
+            ld4(u1, p1 + h);
 #pragma unroll
-                for (int k = 0; k < 4; k++) w[k] = __ldg(R.f1t + (h + k) * 64 + o);
-                ld4(u0, p0 + h);
-                ld4(u1, p1 + h);
+            for (int q = 0; q < 4; q++) {
+                float w[4];
+                ld4(w, F1 + (h + q) * F1_S + o);
 #pragma unroll
-                for (int k = 0; k < 4; k++) { z0 = fmaf(w[k], u0[k], z0); z1 = fmaf(w[k], u1[k], z1); }
-            }
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int ss = 2 * sp + h;
-                float g;
-                const float a = gelu_both<TRAIN>(h ? z1 : z0, g);
-                g1[ss * 64 + o] = a;
-                if (TRAIN && ss < m) {
-                    float *r = R.act + (size_t)(s0 + ss) * REF_ACT;
-                    r[ACT_G1 + o] = a;
-                    r[ACT_DZ + o] = g;
-                }
+                for (int k = 0; k < 4; k++) { z[0][k] = fmaf(w[k], u0[q], z[0][k]); z[1][k] = fmaf(w[k], u1[q], z[1][k]); }
             }
         }
-        __syncthreads();
-        if (tid < 3 * m) {
-            const int ss = tid / 3, o = tid - 3 * ss;
-            float v = P[RP_C2 + o];
-            for (int k = 0; k < 64; k++) v = fmaf(P[RP_F2 + o * 64 + k], g1[ss * 64 + k], v);
-            if (TRAIN) R.act[(size_t)(s0 + ss) * REF_ACT + ACT_OUT + o] = v;
-            if (R.out) R.out[(size_t)(s0 + ss) * 3 + o] = v;
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+            float a[4], g[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) a[k] = gelu_both<TRAIN>(z[b][k], g[k]);
+            const float4 av = make_float4(a[0], a[1], a[2], a[3]);
+            *reinterpret_cast<float4 *>(g1 + (sp + b) * Z_S + o) = av;
+            if (TRAIN) {
+                *reinterpret_cast<float4 *>(dg + (sp + b) * Z_S + o) = make_float4(g[0], g[1], g[2], g[3]);
+                if (sp + b < m) *reinterpret_cast<float4 *>(R.act + (size_t)(s0 + sp + b) * REF_ACT + ACT_G1 + o) = av;
+            }
         }
-        __syncthreads();
     }
-}
-
-// One row of the input gradient of a valid 3x3 convolution for input channels
-// k, k + 1: WO + 2 values each from the WO-wide output-gradient rows
-// i - 2 .. i that exist; weights [c][tap][k].
-template <int WO, int ROWS, int RS>
-__device__ __forceinline__ void conv_back_row(float (&g)[2][WO + 2], const float *dy, int dy_cs, const float *W, int i, int k) {
-    const int d0 = max(0, i - (ROWS - 1)), d1 = min(2, i);
+    __syncthreads();
+    if (tid < 3 * DN_S) {
+        const int ss = tid / 3, o = tid - 3 * ss;
+        float v = P[RP_C2 + o];
+#pragma unroll 8
+        for (int k = 0; k < 64; k++) v = fmaf(F2[o * 64 + k], g1[ss * Z_S + k], v);
+        if (R.out && ss < m) R.out[(size_t)(s0 + ss) * 3 + o] = v;
+        dout[ss * 4 + o] = v;
+    }
+    if (!TRAIN) return;
+    __syncthreads();
+    if (tid < DN_S) {
+        float4 d = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (tid < m) {
+            const int sg = s0 + tid;
+            const float inv_n = 1.0f / (float)n;
+            const float lv = dout[tid * 4 + 2];
+            const float rx = dout[tid * 4] - target[2 * sg], ry = dout[tid * 4 + 1] - target[2 * sg + 1];
+            const float r2 = rx * rx + ry * ry;
+            d.x = rx * inv_n;
+            d.y = ry * inv_n;
+            d.z = (1.0f - 0.5f * r2 * expf(-lv)) * inv_n;
+            if (R.loss) R.loss[sg] = 0.5f * r2 + 0.5f * r2 * expf(-lv) + lv;
+            *reinterpret_cast<float4 *>(R.grad_act + (size_t)sg * REF_GRAD + GRD_OUT) = d;
+        }
+        *reinterpret_cast<float4 *>(dout + tid * 4) = d;
+    }
+    __syncthreads();
+    for (int i = tid; i < DN_S * 64; i += DN_THREADS) {
+        const int ss = i >> 6, o = i & 63;
+        float g = 0.f;
+#pragma unroll
+        for (int e = 0; e < 3; e++) g = fmaf(F2[e * 64 + o], dout[ss * 4 + e], g);
+        const float v = g * dg[ss * Z_S + o];
+        g1[ss * Z_S + o] = v;
+        if (ss < m) R.grad_act[(size_t)(s0 + ss) * REF_GRAD + GRD_Z + o] = v;
+    }
+    __syncthreads();
+    {   // inputs lane + 32 j of samples 4 warp .. 4 warp + 3
+        float g[9][4] = {}, dv[9][4];
+#pragma unroll
+        for (int j = 0; j < 9; j++)
+#pragma unroll
+            for (int b = 0; b < 4; b++)
+                dv[j][b] = 4 * warp + b < m ? R.act[(size_t)(s0 + 4 * warp + b) * REF_ACT + ACT_D3 + lane + 32 * j] : 0.f;
+        const float *dz = g1 + 4 * warp * Z_S;
 #pragma unroll 2
-    for (int c = 0; c < 32; c++) {
-        for (int di = d0; di <= d1; di++) {
-            float v[WO > 4 ? 8 : 4];
-            const float *r = dy + c * dy_cs + (i - di) * RS;
-            ld4(v, r);
-            if constexpr (WO > 4) ld4(v + 4, r + 4);
+        for (int o = 0; o < 64; o += 4) {
+            float d[4][4];
 #pragma unroll
-            for (int dj = 0; dj < 3; dj++) {
-                const float2 w = *reinterpret_cast<const float2 *>(W + (c * 9 + di * 3 + dj) * 32 + k);
+            for (int b = 0; b < 4; b++) ld4(d[b], dz + b * Z_S + o);
 #pragma unroll
-                for (int j = 0; j < WO; j++) {
-                    g[0][j + dj] = fmaf(w.x, v[j], g[0][j + dj]);
-                    g[1][j + dj] = fmaf(w.y, v[j], g[1][j + dj]);
-                }
+            for (int j = 0; j < 9; j++) {
+                float w[4];
+                ld4(w, F1 + (lane + 32 * j) * F1_S + o);
+#pragma unroll
+                for (int b = 0; b < 4; b++)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) g[j][b] = fmaf(w[e], d[b][e], g[j][b]);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 9; j++) {
+            const int h = lane + 32 * j, cc = h / 9, q = h - 9 * cc, at = cc * 12 + (q / 3) * 4 + q % 3;
+#pragma unroll
+            for (int b = 0; b < 4; b++) {
+                const int ss = 4 * warp + b;
+                if (ss < m) R.grad_act[(size_t)(s0 + ss) * REF_GRAD + GRD_Y3 + at] = g[j][b] * dv[j][b];
             }
         }
     }
 }
 
-// Gradients of the loss with respect to every pre-activation, from the
-// outputs back; a task is (sample, input row, two channels).
-constexpr int BWD_THREADS = 896;
-__global__ void __launch_bounds__(BWD_THREADS, 1) k_ref_bwd(RefPlan R, const float *__restrict__ target, int n) {
+// The input gradient of a valid 3x3 convolution of one sample for input channel
+// k: (WO + 2)^2 sums over the WO x WO output gradients of 32 channels dy_cs
+// apart at `dy` (rows RS apart), weights [c][tap][k].
+template <int WO, int RS>
+__device__ __forceinline__ void conv_back_all(float (&g)[WO + 2][WO + 2], const float *dy, int dy_cs, const float *W, int k) {
+#pragma unroll 1
+    for (int c = 0; c < 32; c++) {
+        float w[9];
+#pragma unroll
+        for (int d = 0; d < 9; d++) w[d] = W[(c * 9 + d) * 32 + k];
+#pragma unroll
+        for (int r = 0; r < WO; r++) {
+            float v[WO > 4 ? 8 : 4];
+            ld4(v, dy + c * dy_cs + r * RS);
+            if constexpr (WO > 4) ld4(v + 4, dy + c * dy_cs + r * RS + 4);
+#pragma unroll
+            for (int di = 0; di < 3; di++)
+#pragma unroll
+                for (int dj = 0; dj < 3; dj++)
+#pragma unroll
+                    for (int j = 0; j < WO; j++) g[r + di][j + dj] = fmaf(w[di * 3 + dj], v[j], g[r + di][j + dj]);
+        }
+    }
+}
+
+// The convolutions' input gradients times the GELU derivatives: from conv3's
+// pre-activation gradients to conv2's and conv1's.  Warps 0-3: conv2 of group
+// t - 1, 4-7: conv3 of group t, a warp per sample, a lane per channel; the
+// derivatives are loaded ahead of the sums they multiply.
+constexpr int BWD_THREADS = 256, DY2_LEN = 32 * 40, DY3_LEN = 32 * 12;
+__global__ void __launch_bounds__(BWD_THREADS, 1) k_ref_bwd(RefPlan R, int n) {
     extern __shared__ float4 smem_v[];
     float *W2 = reinterpret_cast<float *>(smem_v);     // [c*9 + tap][k]
     float *W3 = W2 + 9216;
-    float *dy2 = W3 + 9216, *dy3 = dy2 + TR_S * DY2_SS, *dz = dy3 + TR_S * DY3_SS, *dout = dz + TR_S * 64;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float *dy2 = W3 + 9216;                            // [2][TR_S][DY2_LEN] by the group's parity
+    float *dy3 = dy2 + 2 * TR_S * DY2_LEN;             // [2][TR_S][DY3_LEN]
+    float *dy1 = dy3 + 2 * TR_S * DY3_LEN;             // [TR_S][A1_LEN]
+    const int tid = threadIdx.x, k = tid & 31, warp = tid >> 5, s = warp & 3, role = warp >> 2;
+    const int per = (n + gridDim.x - 1) / gridDim.x;
+    const int s_beg = blockIdx.x * per, s_end = min(n, s_beg + per);
+    if (s_beg >= s_end) return;
     for (int i = tid; i < 9216 / 4; i += BWD_THREADS) {
         reinterpret_cast<float4 *>(W2)[i] = reinterpret_cast<const float4 *>(R.w2b)[i];
         reinterpret_cast<float4 *>(W3)[i] = reinterpret_cast<const float4 *>(R.w3b)[i];
     }
-    const float *P = R.theta;
-    const float inv_n = 1.0f / (float)n;
-    const int per = (n + gridDim.x - 1) / gridDim.x;
-    const int s_end = min(n, (int)(blockIdx.x + 1) * per);
-    const int k = 2 * (lane & 15), s = 2 * (warp & 3) + (lane >> 4), row = warp >> 2;
-    for (int s0 = blockIdx.x * per; s0 < s_end; s0 += TR_S) {
-        const int m = min(TR_S, s_end - s0);
-        const bool have = s < m;
-        const float *rec = R.act + (size_t)(s0 + (have ? s : 0)) * REF_ACT;
-        float *gr = R.grad_act + (size_t)(s0 + (have ? s : 0)) * REF_GRAD;
-        __syncthreads();
-        if (tid < TR_S) {
-            float d[3] = {0.f, 0.f, 0.f};
-            if (tid < m) {
-                const int sg = s0 + tid;
-                const float *o = R.act + (size_t)sg * REF_ACT + ACT_OUT;
-                const float lv = o[2];
-                const float rx = o[0] - target[2 * sg], ry = o[1] - target[2 * sg + 1];
-                const float r2 = rx * rx + ry * ry;
-                d[0] = rx * inv_n;
-                d[1] = ry * inv_n;
-                d[2] = (1.0f - 0.5f * r2 * expf(-lv)) * inv_n;
-                if (R.loss) R.loss[sg] = 0.5f * r2 + 0.5f * r2 * expf(-lv) + lv;
-                float *g = R.grad_act + (size_t)sg * REF_GRAD;
-                g[GRD_OUT] = d[0]; g[GRD_OUT + 1] = d[1]; g[GRD_OUT + 2] = d[2]; g[GRD_OUT + 3] = 0.f;
-            }
+    const int groups = (s_end - s_beg + TR_S - 1) / TR_S;
+    // conv3's warps copy their sample's gradients ahead, a group at a time
+    auto fetch = [&](int g) {
+        const int at = s_beg + g * TR_S + s;
+        if (at < s_end)
 #pragma unroll
-            for (int o = 0; o < 3; o++) dout[tid * 4 + o] = d[o];
-        }
-        __syncthreads();
-        if (tid < TR_S * 64) {
-            const int ss = tid >> 6, o = tid & 63;
-            float v = 0.f;
-            if (ss < m) {
-                float g = 0.f;
+            for (int q = 0; q < 3; q++)
+                cp_async16(dy3 + ((g & 1) * TR_S + s) * DY3_LEN + 4 * (k + 32 * q),
+                           R.grad_act + (size_t)at * REF_GRAD + GRD_Y3 + 4 * (k + 32 * q));
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    if (role == 1) fetch(0);
+    __syncthreads();
+    for (int t = 0; t < groups + 1; t++) {
+        const int g = t - (role == 0 ? 1 : 0);
+        const int at = s_beg + g * TR_S + s;
+        const bool have = g >= 0 && g < groups && at < s_end;
+        const float *rec = R.act + (size_t)(have ? at : s_beg) * REF_ACT;
+        float *gr = R.grad_act + (size_t)(have ? at : s_beg) * REF_GRAD;
+        const int buf = g & 1;
+        if (role == 1) {
+            fetch(g + 1);
+            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+            __syncwarp();
+            if (have) {
+                float d[5][8], a[5][5] = {};
 #pragma unroll
-                for (int e = 0; e < 3; e++) g = fmaf(P[RP_F2 + e * 64 + o], dout[ss * 4 + e], g);
-                v = g * R.act[(size_t)(s0 + ss) * REF_ACT + ACT_DZ + o];
-                R.grad_act[(size_t)(s0 + ss) * REF_GRAD + GRD_Z + o] = v;
-            }
-            dz[tid] = v;
-        }
-        __syncthreads();
-        if (tid < 864) {                               // dense input gradient: h of a third of the samples
-            const int h = tid % 288, t3 = tid / 288;
-            const int b0 = 3 * t3, nb = t3 == 2 ? 2 : 3;
-            float g[3] = {0.f, 0.f, 0.f};
-#pragma unroll 4
-            for (int o = 0; o < 64; o += 4) {
-                float w[4];
+                for (int i = 0; i < 5; i++) { ld4(d[i], rec + ACT_D2 + k * 40 + i * 8); ld4(d[i] + 4, rec + ACT_D2 + k * 40 + i * 8 + 4); }
+                conv_back_all<3, 4>(a, dy3 + (buf * TR_S + s) * DY3_LEN, 12, W3, k);
+                float *out = dy2 + (buf * TR_S + s) * DY2_LEN + k * 40;
 #pragma unroll
-                for (int e = 0; e < 4; e++) w[e] = __ldg(P + RP_F1 + (o + e) * 288 + h);
-#pragma unroll
-                for (int b = 0; b < 3; b++) {
-                    if (b >= nb) break;
-                    float d[4];
-                    ld4(d, dz + (b0 + b) * 64 + o);
-#pragma unroll
-                    for (int e = 0; e < 4; e++) g[b] = fmaf(w[e], d[e], g[b]);
+                for (int i = 0; i < 5; i++) {
+                    *reinterpret_cast<float4 *>(out + i * 8) =
+                        make_float4(a[i][0] * d[i][0], a[i][1] * d[i][1], a[i][2] * d[i][2], a[i][3] * d[i][3]);
+                    *reinterpret_cast<float4 *>(out + i * 8 + 4) = make_float4(a[i][4] * d[i][4], 0.f, 0.f, 0.f);
                 }
             }
-            const int c = h / 9, p = h - 9 * c, at = c * 12 + (p / 3) * 4 + p % 3;
-            for (int b = 0; b < nb; b++) {
-                const int ss = b0 + b;
-                if (ss >= m) break;
-                const float v = g[b] * R.act[(size_t)(s0 + ss) * REF_ACT + ACT_D3 + h];
-                dy3[ss * DY3_SS + at] = v;
-                R.grad_act[(size_t)(s0 + ss) * REF_GRAD + GRD_Y3 + at] = v;
+        } else if (have) {
+            float d[7][8], a[7][7] = {};
+#pragma unroll
+            for (int i = 0; i < 7; i++) { ld4(d[i], rec + ACT_D1 + k * 56 + i * 8); ld4(d[i] + 4, rec + ACT_D1 + k * 56 + i * 8 + 4); }
+            conv_back_all<5, 8>(a, dy2 + (buf * TR_S + s) * DY2_LEN, 40, W2, k);
+            if (k == 0) bulk_wait_read<0>();           // the sample before has left this warp's rows
+            __syncwarp();
+            float *out = dy1 + s * A1_LEN + k * A1_CS;
+#pragma unroll
+            for (int i = 0; i < 7; i++) {
+                *reinterpret_cast<float4 *>(out + i * 8) =
+                    make_float4(a[i][0] * d[i][0], a[i][1] * d[i][1], a[i][2] * d[i][2], a[i][3] * d[i][3]);
+                *reinterpret_cast<float4 *>(out + i * 8 + 4) = make_float4(a[i][4] * d[i][4], a[i][5] * d[i][5], a[i][6] * d[i][6], 0.f);
             }
+            fence_bulk();
+            __syncwarp();
+            if (k == 0) { bulk_out(gr + GRD_Y1, dy1 + s * A1_LEN, A1_LEN * 4); bulk_commit(); }
+        }
+        if (role == 1) {
+            if (k == 0) bulk_wait_read<0>();           // this warp's copy of the step before
+            fence_bulk();
         }
         __syncthreads();
-        if (have && row < 5) {                         // conv3's input gradient
-            float g[2][5] = {};
-            conv_back_row<3, 3, 4>(g, dy3 + s * DY3_SS, 12, W3, row, k);
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                float v[8], d[8];
-                ld4(d, rec + ACT_D2 + (k + h) * 40 + row * 8);
-                ld4(d + 4, rec + ACT_D2 + (k + h) * 40 + row * 8 + 4);
-#pragma unroll
-                for (int j = 0; j < 8; j++) v[j] = j < 5 ? g[h][j < 5 ? j : 0] * d[j] : 0.f;
-#pragma unroll
-                for (int u = 0; u < 2; u++) {
-                    const float4 o = make_float4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
-                    *reinterpret_cast<float4 *>(dy2 + s * DY2_SS + (k + h) * 40 + row * 8 + 4 * u) = o;
-                    *reinterpret_cast<float4 *>(gr + GRD_Y2 + (k + h) * 40 + row * 8 + 4 * u) = o;
-                }
-            }
-        }
-        __syncthreads();
-        if (have) {                                    // conv2's input gradient
-            float g[2][7] = {};
-            conv_back_row<5, 5, 8>(g, dy2 + s * DY2_SS, 40, W2, row, k);
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                float v[8], d[8];
-                ld4(d, rec + ACT_D1 + (k + h) * 56 + row * 8);
-                ld4(d + 4, rec + ACT_D1 + (k + h) * 56 + row * 8 + 4);
-#pragma unroll
-                for (int j = 0; j < 8; j++) v[j] = j < 7 ? g[h][j < 7 ? j : 0] * d[j] : 0.f;
-#pragma unroll
-                for (int u = 0; u < 2; u++)
-                    *reinterpret_cast<float4 *>(gr + GRD_Y1 + (k + h) * A1_CS + row * 8 + 4 * u) =
-                        make_float4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
-            }
-        }
+        if (role == 1 && k == 0 && have) { bulk_out(gr + GRD_Y2, dy2 + (buf * TR_S + s) * DY2_LEN, DY2_LEN * 4); bulk_commit(); }
     }
+    if (k == 0) bulk_wait_all();
 }
 
 // ---------------------------------------------------------------- parameter gradients
@@ -787,29 +865,38 @@ __global__ void __launch_bounds__(128 * INF_GROUPS) k_ref_infer(RefPlan R, const
     }
 }
 
-size_t ref_fwd_smem() { return (size_t)(2 * 9216 + TR_S * (X0_S + A1_SS + A2_SS + A3_SS + 64)) * sizeof(float); }
-size_t ref_bwd_smem() { return (size_t)(2 * 9216 + TR_S * (DY2_SS + DY3_SS + 64 + 4)) * sizeof(float); }
+size_t ref_fwd_smem() { return (size_t)(2 * 9216 + TR_S * (2 * (A1_LEN + A2_LEN) + X0_S)) * sizeof(float); }
+size_t ref_dense_smem() { return (size_t)(288 * F1_S + DN_S * (A3_SS + 2 * Z_S + 4) + 192) * sizeof(float); }
+size_t ref_bwd_smem() { return (size_t)(2 * 9216 + TR_S * (2 * (DY2_LEN + DY3_LEN) + A1_LEN)) * sizeof(float); }
 size_t ref_wgrad_smem() { return (size_t)2 * WS_LEN * sizeof(float); }
 size_t ref_infer_smem() { return (size_t)INF_PACK_BYTES + (size_t)INF_GROUPS * INF_ACT_BYTES; }
 
 cudaError_t ref_setup() {
     cudaError_t e = cudaFuncSetAttribute(k_ref_fwd<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ref_fwd_smem());
     if (!e) e = cudaFuncSetAttribute(k_ref_fwd<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ref_fwd_smem());
+    if (!e) e = cudaFuncSetAttribute(k_ref_dense<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ref_dense_smem());
+    if (!e) e = cudaFuncSetAttribute(k_ref_dense<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ref_dense_smem());
     if (!e) e = cudaFuncSetAttribute(k_ref_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ref_bwd_smem());
     if (!e) e = cudaFuncSetAttribute(k_ref_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ref_wgrad_smem());
     if (!e) e = cudaFuncSetAttribute(k_ref_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ref_infer_smem());
     return e;
 }
 
-// CTAs of the forward and backward kernels: a group of eight samples each
+// CTAs of the forward and backward kernels: a group of four samples each
 // until every SM has one, then longer ranges
 static int train_grid(int n) { return std::min((n + TR_S - 1) / TR_S, REF_SMS); }
-void ref_launch_fwd(const RefPlan &R, const float *feat, int n, bool train, cudaStream_t s) {
-    if (train) k_ref_fwd<true><<<train_grid(n), FWD_THREADS, ref_fwd_smem(), s>>>(R, feat, n);
-    else k_ref_fwd<false><<<train_grid(n), FWD_THREADS, ref_fwd_smem(), s>>>(R, feat, n);
+void ref_launch_fwd(const RefPlan &R, const float *feat, const float *target, int n, cudaStream_t s) {
+    const int dense = (n + DN_S - 1) / DN_S;
+    if (target) {
+        k_ref_fwd<true><<<train_grid(n), FWD_THREADS, ref_fwd_smem(), s>>>(R, feat, n);
+        k_ref_dense<true><<<dense, DN_THREADS, ref_dense_smem(), s>>>(R, target, n);
+    } else {
+        k_ref_fwd<false><<<train_grid(n), FWD_THREADS, ref_fwd_smem(), s>>>(R, feat, n);
+        k_ref_dense<false><<<dense, DN_THREADS, ref_dense_smem(), s>>>(R, nullptr, n);
+    }
 }
-void ref_launch_bwd(const RefPlan &R, const float *target, int n, cudaStream_t s) {
-    k_ref_bwd<<<train_grid(n), BWD_THREADS, ref_bwd_smem(), s>>>(R, target, n);
+void ref_launch_bwd(const RefPlan &R, int n, cudaStream_t s) {
+    k_ref_bwd<<<train_grid(n), BWD_THREADS, ref_bwd_smem(), s>>>(R, n);
 }
 // partial gradient vectors of a batch of n: at least four samples each, one per SM at most
 int ref_wgrad_parts(int n) { return std::min((n + 3) / 4, REF_SMS); }

@@ -46,9 +46,11 @@ struct RefPlan {
 };
 
 cudaError_t ref_setup();
-// train: keep what the backward kernels read in the samples' records
-void ref_launch_fwd(const RefPlan &R, const float *feat, int n, bool train, cudaStream_t s);
-void ref_launch_bwd(const RefPlan &R, const float *target, int n, cudaStream_t s);
+// The forward pass of n samples; with target also the loss and the gradients
+// back to the last convolution, everything the backward kernels read kept in
+// the samples' records.
+void ref_launch_fwd(const RefPlan &R, const float *feat, const float *target, int n, cudaStream_t s);
+void ref_launch_bwd(const RefPlan &R, int n, cudaStream_t s);
 int ref_wgrad_parts(int n);
 void ref_launch_wgrad(const RefPlan &R, const float *feat, int n, cudaStream_t s);
 void ref_launch_adam(const RefPlan &R, float lr, int step, cudaStream_t s);

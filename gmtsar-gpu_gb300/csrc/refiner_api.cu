@@ -111,7 +111,7 @@ xcg_status xcg_refiner_forward(xcg_refiner *r, const float *d_feat, int32_t n, f
             R.out = d_out + (size_t)c0 * 3;
             R.loss = nullptr;
             const int m = (n - c0 < r->max_batch) ? n - c0 : r->max_batch;
-            xcg::ref_launch_fwd(R, d_feat + (size_t)c0 * 81, m, false, s);
+            xcg::ref_launch_fwd(R, d_feat + (size_t)c0 * 81, nullptr, m, s);
         }
     }
     return ck(cudaGetLastError(), "refiner forward");
@@ -120,8 +120,8 @@ xcg_status xcg_refiner_forward(xcg_refiner *r, const float *d_feat, int32_t n, f
 static void run_grad(xcg_refiner *r, const float *d_feat, const float *d_target, int n, cudaStream_t s) {
     xcg::RefPlan R = r->R;
     R.out = r->out_int;
-    xcg::ref_launch_fwd(R, d_feat, n, true, s);
-    xcg::ref_launch_bwd(R, d_target, n, s);
+    xcg::ref_launch_fwd(R, d_feat, d_target, n, s);
+    xcg::ref_launch_bwd(R, n, s);
     xcg::ref_launch_wgrad(R, d_feat, n, s);
 }
 
