@@ -111,9 +111,10 @@ inline void launch_chain(const Plan &P, Kernel kern, dim3 grid, int threads, siz
 //              transforms up to 256 points), 3 for 512 points; 1: one fewer
 #define XCG_COLS_BLOCKS 5
 
-template <int M, int THR = 128>
+// LANES: lanes of a column's team
+template <int M, int THR = 128, int LANES = fft_lanes(M)>
 struct ColsGeom {
-    static constexpr int T = fft_lanes(M);
+    static constexpr int T = LANES;
     static constexpr int PADM = fft_padded_len(M);
     static constexpr int THREADS = THR;
     static constexpr int CP = THREADS / T;        // column pairs per CTA = teams

@@ -733,11 +733,17 @@ __global__ void __launch_bounds__(THR, ColsGeom<M, THR>::BLOCKS) k_cols_rc(Plan 
 // packed DC/Nyquist column, whose second output goes through the slave slot)
 // request the next tile's slave rows only after their copy-out.
 // KEEP: the slave's column spectrum stays in registers for the product
-// (one CTA per SM fewer; the default form up to 256-point columns).
-template <int M, int THR, bool KEEP>
-__global__ void __launch_bounds__(THR, KEEP ? ColsGeom<M, THR>::BLOCKS - 1 : ColsGeom<M, THR>::BLOCKS)
-k_cols_rcp(Plan P) {
-    using G = ColsGeom<M, THR>;
+// (the default form up to 512-point columns).  LANES: lanes of a column's team;
+// MINB: CTAs per SM.
+//
+// 512-point columns go to teams of 16 lanes with 32 elements each: the
+// exchanges through shared memory bound this kernel, and such a team needs one
+// per transform where 32 lanes need two.  The registers leave two CTAs per SM
+// (205 a thread).  40,000 patches of 512 x 512: 31.2 ms, without the slave's
+// spectrum in registers 32.3, with 32 lanes at three CTAs per SM 37.7.
+template <int M, int THR, bool KEEP, int LANES, int MINB>
+__global__ void __launch_bounds__(THR, MINB) k_cols_rcp(Plan P) {
+    using G = ColsGeom<M, THR, LANES>;
     constexpr int T = G::T, CS = G::CS, CP = G::CP, TWL = G::TWL;
     constexpr int PER = M / T;
     constexpr int RSTEP = THR / CP;            // rows a staging pass covers
@@ -870,7 +876,7 @@ k_cols_rcp(Plan P) {
         for (int m = 0; m < PER; m++)
             z[m] = (m >= PER / 4 && m < 3 * PER / 4) ? pa[fft_pad(lane + T * m)] : make_float2(0.f, 0.f);
         __syncwarp();
-        team_fft_reg_mid<M, -1>(z, pa, tw, lane);    // zero outside the mask rows
+        team_fft_reg_mid<M, -1, T>(z, pa, tw, lane);    // zero outside the mask rows
         float2 zs[KEEP ? PER : 1];
         if constexpr (KEEP) {
 #pragma unroll
@@ -886,7 +892,7 @@ k_cols_rcp(Plan P) {
 #pragma unroll
         for (int m = 0; m < PER; m++) z[m] = a[fft_pad(lane + T * m)];
         __syncwarp();
-        team_fft_reg<M, -1>(z, a, tw, lane);
+        team_fft_reg<M, -1, T>(z, a, tw, lane);
 
         auto product = [&](int kxx, float2 A1, float2 A2, int ky) {
             if (kxx == 0 && ky == 0) A1.x -= dc1;
@@ -947,7 +953,7 @@ k_cols_rcp(Plan P) {
             }
             float2 *dst = (o == 0) ? a : pa;
             __syncwarp();
-            team_fft_reg<M, +1>(z, dst, tw, lane);
+            team_fft_reg<M, +1, T>(z, dst, tw, lane);
 #pragma unroll
             for (int m = PER / 4; m < 3 * PER / 4; m++) dst[fft_pad(lane + T * m)] = z[m];
             __syncwarp();
@@ -995,9 +1001,9 @@ static size_t segrows_smem() {
            (size_t)teams * (fft_padded_len(N) * sizeof(float2) + (2 * N + 32) * sizeof(float)) +
            (LG >= 2 ? (size_t)128 * (N / T) * sizeof(float2) : (size_t)(128 / 32) * (ACC + 32) * sizeof(float));
 }
-template <int M>
+template <int M, int LANES = fft_lanes(M)>
 static size_t cols_rc_smem() {
-    using G = ColsGeom<M, 128>;
+    using G = ColsGeom<M, 128, LANES>;
     return G::TWL * sizeof(float2) + (size_t)(2 * G::CP + 1) * G::CS * sizeof(float2) +
            (size_t)(M + G::CP + 1) * sizeof(float2) + 4 * sizeof(double) + 16;
 }
@@ -1014,16 +1020,36 @@ static cudaError_t setup_segrows_t() {
     set(k_segrows<N, 3>, segrows_smem<N, 3>());
     return e;
 }
+// The persistent column stage in a form: WIDE (512 points: 16 lanes per
+// column) or not, the slave's spectrum kept in registers or not (at one CTA
+// per SM fewer).
+template <int M, bool WIDE, bool KEEP>
+struct ColsForm {
+    static constexpr int LANES = WIDE ? 16 : fft_lanes(M);
+    static constexpr int MINB = WIDE ? 2 : (KEEP ? ColsGeom<M, 128>::BLOCKS - 1 : ColsGeom<M, 128>::BLOCKS);
+    static constexpr int CP = ColsGeom<M, 128, LANES>::CP;
+    static size_t smem() { return cols_rc_smem<M, LANES>(); }
+    static auto kernel() { return k_cols_rcp<M, 128, KEEP, LANES, MINB>; }
+    static cudaError_t setup() {
+        return cudaFuncSetAttribute(kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem());
+    }
+    static void launch(const Plan &P, int sms, cudaStream_t s) {
+        const int ntiles = (P.npx / 2) / CP * P.nwin;
+        launch_chain(P, kernel(), dim3(std::min(ntiles, sms * MINB)), 128, smem(), s);
+    }
+};
+// the default form of a size and the one launch shape 2 takes
+template <int M>
+struct ColsForms {
+    using Default = ColsForm<M, M == 512, (M <= 512)>;
+    using Other = ColsForm<M, false, (M >= 1024)>;
+};
 template <int M>
 static cudaError_t setup_cols_rc_t() {
     cudaError_t e = cudaFuncSetAttribute(k_cols_rc<M, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)cols_rc_smem<M>());
-    if (e) return e;
-    e = cudaFuncSetAttribute(k_cols_rcp<M, 128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)cols_rc_smem<M>());
-    if (e) return e;
-    return cudaFuncSetAttribute(k_cols_rcp<M, 128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)cols_rc_smem<M>());
+    if (!e) e = ColsForms<M>::Default::setup();
+    return e ? e : ColsForms<M>::Other::setup();
 }
 
 cudaError_t segrows_setup(const Plan &P) {
@@ -1096,30 +1122,19 @@ void launch_segrows(const Plan &P, cudaStream_t s) {
 template <int M>
 static void launch_cols_rc_t(const Plan &P, cudaStream_t s) {
     using G = ColsGeom<M, 128>;
-    const int ntiles = ((P.npx / 2) / G::CP) * P.nwin;
     if (P.cols_cfg == 1) {                       // one CTA per tile
         dim3 grid((P.npx / 2) / G::CP, P.nwin);
         k_cols_rc<M, 128><<<grid, 128, cols_rc_smem<M>(), s>>>(P);      // (not a dependent: it does not wait)
         return;
     }
-    // persistent: one CTA per resident slot, tiles split into contiguous
-    // ranges (leaving one slot per SM to the other batch's kernels measured
-    // the same on the device entry and slower on the host entry)
+    // persistent: one CTA per resident slot, tiles from a counter (leaving
+    // one slot per SM to the other batch's kernels measured the same on the
+    // device entry and slower on the host entry)
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    // the slave spectrum kept in registers (one CTA per SM fewer): the
-    // default up to 256 points (0.454 against 0.481 ms per 1000 windows of
-    // 128 x 128), not beyond (full frame 72.4 against 69.5 ms); launch
-    // shape 2 takes the other form
-    const bool keep = (P.cols_cfg == 2) != (M <= 256);
-    if (keep && G::BLOCKS > 1) {
-        const int grid = std::min(ntiles, sms * (G::BLOCKS - 1));
-        launch_chain(P, k_cols_rcp<M, 128, true>, dim3(grid), 128, cols_rc_smem<M>(), s);
-        return;
-    }
-    const int grid = std::min(ntiles, sms * G::BLOCKS);
-    launch_chain(P, k_cols_rcp<M, 128, false>, dim3(grid), 128, cols_rc_smem<M>(), s);
+    if (P.cols_cfg == 2) ColsForms<M>::Other::launch(P, sms, s);
+    else ColsForms<M>::Default::launch(P, sms, s);
 }
 void launch_cols_rc(const Plan &P, cudaStream_t s) {
     switch (P.npy) {

@@ -298,16 +298,22 @@ __host__ __device__ constexpr float sin32(int k) { return cos32(k - 8); }
 // ZMID: the sequence is zero outside registers [N/T/4, 3N/T/4), i.e. outside
 // elements [N/4, 3N/4) (a masked column); the first pass then skips the
 // butterflies with a zero input (its 16-point DFTs see elements [4, 12) only).
-template <int N, int DIR, int PASS, bool HS = false, bool ZMID = false>
+// T: lanes of the team; fft_lanes(N) (16 elements per lane up to 512 points),
+// or 16 lanes of 32 elements for N = 512: a lane then holds the outputs of the
+// second pass's butterflies j and j + 16, which are what its radix-2 third
+// pass combines, so one exchange remains of two.  The same operations on the
+// same elements, so the same bits.
+template <int N, int DIR, int PASS, bool HS = false, bool ZMID = false, int T = fft_lanes(N)>
 __device__ __forceinline__ void team_fft_reg_pass(float2 *v, float2 *ex, const float2 *tw, int Ns, int lane) {
-    constexpr int T = fft_lanes(N);
+    constexpr bool WIDE512 = (N == 512 && T == 16);
     constexpr int NP = fft_npasses(N);
     constexpr int R = fft_radix(N, PASS);
     constexpr int NR = N / R;
     constexpr int IT = NR / T;                 // butterflies per lane in this pass
     static_assert(IT * R * T == N, "team layout");
-    static_assert(!HS || (DIR > 0 && N / T == 16 && IT == 1 && (NP == 2 || N == 512)),
+    static_assert(!HS || (DIR > 0 && ((N / T == 16 && IT == 1) || WIDE512) && (NP == 2 || N == 512)) || PASS > 0,
                   "half-sample shift: N = 128, 256 or 512");
+    static_assert(T == fft_lanes(N) || WIDE512, "lanes of a team");
     static_assert(!ZMID || (fft_radix(N, 0) == 16 && !HS), "zero outside the middle half: radix-16 first pass");
     if constexpr (PASS == 0) {
         // inputs from registers: element (lane + T*it) + NR*r = lane + T*(it + r*IT)
@@ -331,7 +337,7 @@ __device__ __forceinline__ void team_fft_reg_pass(float2 *v, float2 *ex, const f
             for (int r = 0; r < R; r++) ex[fft_pad(j * R + r)] = u[r];
         }
         __syncwarp();
-        team_fft_reg_pass<N, DIR, 1>(v, ex, tw, R, lane);
+        team_fft_reg_pass<N, DIR, 1, false, false, T>(v, ex, tw, R, lane);
     } else if constexpr (PASS < NP) {
         float2 u[IT][R];
 #pragma unroll
@@ -349,7 +355,18 @@ __device__ __forceinline__ void team_fft_reg_pass(float2 *v, float2 *ex, const f
         if constexpr (PASS < NP - 1) __syncwarp();
 #pragma unroll
         for (int it = 0; it < IT; it++) dft_reg<R, DIR>(u[it]);
-        if constexpr (PASS == NP - 1) {
+        if constexpr (WIDE512) {
+            // butterfly lane + 16 r of the last pass: outputs r of this lane's two
+            const float2 *tw2 = tw + (R - 1) * Ns;
+#pragma unroll
+            for (int r = 0; r < 16; r++) {
+                const float2 w = tw2[lane + 16 * r];
+                float2 p[2] = {u[0][r], DIR < 0 ? cmulf(u[1][r], w) : cmulf_conj(u[1][r], w)};
+                dft_reg<2, DIR>(p);
+                v[r] = p[0];
+                v[r + 16] = p[1];
+            }
+        } else if constexpr (PASS == NP - 1) {
             // last pass: element j + Ns*r with j = lane + T*it and Ns = NR -> register it + r*IT
 #pragma unroll
             for (int it = 0; it < IT; it++)
@@ -365,7 +382,7 @@ __device__ __forceinline__ void team_fft_reg_pass(float2 *v, float2 *ex, const f
                 for (int r = 0; r < R; r++) ex[fft_pad((j - k) * R + k + r * Ns)] = u[it][r];
             }
             __syncwarp();
-            team_fft_reg_pass<N, DIR, PASS + 1>(v, ex, tw + (R - 1) * Ns, Ns * R, lane);
+            team_fft_reg_pass<N, DIR, PASS + 1, false, false, T>(v, ex, tw + (R - 1) * Ns, Ns * R, lane);
         }
     }
 }
@@ -373,22 +390,22 @@ __device__ __forceinline__ void team_fft_reg_pass(float2 *v, float2 *ex, const f
 // In-register N-point FFT of the team's sequence v (N/T values per lane).
 // ex: the team's exchange buffer, fft_padded_len(N) entries.  tw: the
 // size-N pass twiddle table.  All lanes of the warp must call it.
-template <int N, int DIR>
+template <int N, int DIR, int T = fft_lanes(N)>
 __device__ __forceinline__ void team_fft_reg(float2 *v, float2 *ex, const float2 *tw, int lane) {
-    team_fft_reg_pass<N, DIR, 0>(v, ex, tw, 1, lane);
+    team_fft_reg_pass<N, DIR, 0, false, false, T>(v, ex, tw, 1, lane);
 }
 
 // The same for a sequence that is zero outside elements [N/4, 3N/4).
-template <int N, int DIR>
+template <int N, int DIR, int T = fft_lanes(N)>
 __device__ __forceinline__ void team_fft_reg_mid(float2 *v, float2 *ex, const float2 *tw, int lane) {
-    team_fft_reg_pass<N, DIR, 0, false, true>(v, ex, tw, 1, lane);
+    team_fft_reg_pass<N, DIR, 0, false, true, T>(v, ex, tw, 1, lane);
 }
 
 // Inverse FFT of X[f] * exp(i pi f' / N) / N (the odd samples of a 2x
 // zero-pad interpolation) for N = 128, 256 or 512; twh: the tables put_row_phase builds.
-template <int N>
+template <int N, int T = fft_lanes(N)>
 __device__ __forceinline__ void team_ifft_half_shift(float2 *v, float2 *ex, const float2 *twh, int lane) {
-    team_fft_reg_pass<N, +1, 0, true>(v, ex, twh, 1, lane);
+    team_fft_reg_pass<N, +1, 0, true, false, T>(v, ex, twh, 1, lane);
 }
 
 }  // namespace xcg
