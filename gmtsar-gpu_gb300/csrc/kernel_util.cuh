@@ -76,8 +76,15 @@ __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol
 // so the next kernel starts when the last CTA of this one leaves; what is saved
 // is the launch: 1000 windows 401 -> 395 us, through host buffers 578 -> 566.
 // (Starting it during the last tile measured the same.)
+// A batch alone also asks for the largest shared-memory split from its first
+// kernel (dependent = false) on: an SM changes its split only when it is idle,
+// so a kernel of another split could not start beside the one before it (the
+// strip: 51.8 -> 48.4 us).  With several batches the same split would mix their
+// row and column kernels on an SM, which costs (40,000 windows of 256 x 256:
+// 54.8 -> 61.8 ms), so they keep the splits of their own sizes.
 template <class Kernel>
-inline void launch_chain(const Plan &P, Kernel kern, dim3 grid, int threads, size_t smem, cudaStream_t s, int cluster = 1) {
+inline void launch_chain(const Plan &P, Kernel kern, dim3 grid, int threads, size_t smem, cudaStream_t s, int cluster = 1,
+                         bool dependent = true) {
     if (!P.chain && cluster == 1) {
         kern<<<grid, threads, smem, s>>>(P);
         return;
@@ -87,9 +94,13 @@ inline void launch_chain(const Plan &P, Kernel kern, dim3 grid, int threads, siz
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute at[2];
+    cudaLaunchAttribute at[3];
     cfg.attrs = at;
-    if (P.chain) {
+    if (P.chain == 1) {
+        at[cfg.numAttrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        at[cfg.numAttrs++].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
+    }
+    if (P.chain && dependent) {
         at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
     }

@@ -302,6 +302,49 @@ __global__ void __launch_bounds__(NT, 1) k_rc_plan(Plan P) {
 template <int N, int LG>
 __host__ __device__ constexpr int segrows_twiddles() { return (N <= 512 && LG < 2) ? 2 * fft_twiddle_len(N) : fft_twiddle_len(N); }
 
+// row buffer of a team in shared memory: two rows of amplitudes in natural
+// order, padded (factor 1 keeps them in registers)
+__host__ __device__ constexpr int segrows_rowbuf(int n, int lg) { return lg == 0 ? 0 : 2 * n + 32; }
+
+// Sum over the warp of t[m] at index (lane / T) (PER T) + lane % T + T m, in the
+// tree order of h_reduceFD_strip (strides halving from the top).  A level whose
+// stride is a lane distance leaves each lane half of its values: it sends the
+// other half, and the next index bit takes the lane bit's place, so PER values
+// cost PER shuffles however many lanes the top levels span.
+template <int T, int PER>
+__device__ __forceinline__ float chunk_tree(float (&t)[PER], int l32) {
+    constexpr int C = (T == 32) ? 0 : (T == 16) ? 1 : (T == 8) ? 2 : 3;      // index bits above a team
+    constexpr int LEVELS = C + ((PER == 32) ? 5 : 4);
+    static_assert((T << C) == 32 && (PER == 16 || PER == 32), "layout of the sums");
+#pragma unroll
+    for (int i = 0; i < LEVELS; i++) {
+        const int half = (PER >> i) / 2, bit = C ? 16 >> (i % (C ? C : 1)) : 0;
+        if (C == 0) {
+#pragma unroll
+            for (int q = 0; q < half; q++) t[q] = t[q] + t[q + half];
+        } else if (half >= 1) {
+            const bool hi = (l32 & bit) != 0;
+#pragma unroll
+            for (int q = 0; q < half; q++) {
+                const float mine = hi ? t[q + half] : t[q], other = hi ? t[q] : t[q + half];
+                t[q] = mine + __shfl_xor_sync(0xffffffffu, other, bit);
+            }
+        } else {
+            t[0] = t[0] + __shfl_xor_sync(0xffffffffu, t[0], bit);
+        }
+    }
+    float x = t[0];
+#pragma unroll
+    for (int o = T / 2; o > 0; o >>= 1) x = x + __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+
+// Shared-memory wavefronts bound it (88% of the pipe at 512 points, 61% of the
+// issue slots), so what a lane can get by shuffles does not go through memory:
+// the last pass of a 512-point transform, the mirrored element of the two rows'
+// split and the chunk's sum (40,000 patches of 512 x 512: 17.1 -> 15.6 ms; 1000
+// of 256 x 256: 156 -> 151 us).
+//
 // One warp per chunk of rows of one image segment; the structure of k_rows
 // (teams of T lanes, the rows t and t + 512 of the chunk through one team,
 // rows in registers in the team layout) with one image instead of a window's
@@ -316,13 +359,12 @@ __global__ void __launch_bounds__(128, (N >= 1024) ? 2 : (N >= 512 ? 3 : 4)) k_s
     constexpr int RPC = (N >= 1024) ? 1 : 1024 / N;
     constexpr int RPT = (N >= 1024) ? 1 : 2;
     static_assert(RPT * TPW == RPC, "chunk rows");
-    constexpr int ACC = (N >= 1024) ? 1024 : 512;
     constexpr int TWL = fft_twiddle_len(N);
     constexpr int PER = N / T;
     constexpr int NH = N / 2;
     constexpr bool HSHIFT = (LG == 1) && (N <= 512);
     constexpr int TWS = segrows_twiddles<N, LG>();
-    constexpr int RBP = 32;
+    constexpr int RBF = segrows_rowbuf(N, LG);
     constexpr int GOFF = 32 / TPW;
     constexpr bool KEEPS = LG >= 2;                     // the row's spectrum is kept for the phases after the first
 
@@ -332,20 +374,17 @@ __global__ void __launch_bounds__(128, (N >= 1024) ? 2 : (N >= 512 ? 3 : 4)) k_s
     const int lane = l32 % T;
     const int tm = l32 / T;
     const int team = warp * TPW + tm;
-    char *tbase = reinterpret_cast<char *>(tw + TWS) + (size_t)team * (PADN * sizeof(float2) + (2 * N + RBP) * sizeof(float));
+    char *tbase = reinterpret_cast<char *>(tw + TWS) + (size_t)team * (PADN * sizeof(float2) + RBF * sizeof(float));
     float2 *ex = reinterpret_cast<float2 *>(tbase);
     float *rb = reinterpret_cast<float *>(ex + PADN) + tm * GOFF;
     const int rbx = tm & 1;
     float *const rbE = rb + rbx, *const rbO = rb - rbx;
     float *const rbL = (lane & 1) ? rbO : rbE;
+    float ar[(LG == 0) ? RPT : 1][PER];                 // factor 1: the amplitudes of the team's rows
     char *after = reinterpret_cast<char *>(tw + TWS) +
-                  (size_t)(blockDim.x / T) * (PADN * sizeof(float2) + (2 * N + RBP) * sizeof(float));
-    // KEEPS: each thread's spectrum elements, [PER][32] per warp; the warp's
-    // first-level sums use the same memory once its rows are interpolated
+                  (size_t)(blockDim.x / T) * (PADN * sizeof(float2) + RBF * sizeof(float));
+    // KEEPS: each thread's spectrum elements, [PER][32] per warp
     float2 *spec = reinterpret_cast<float2 *>(after) + (size_t)warp * PER * 32 + l32;
-    static_assert(!KEEPS || (ACC + RBP) * sizeof(float) <= PER * 32 * sizeof(float2), "sums fit the spectra");
-    float *acc = KEEPS ? reinterpret_cast<float *>(spec - l32)
-                       : reinterpret_cast<float *>(after) + (size_t)warp * (ACC + RBP);   // [ACC + RBP] first-level sums of the warp's chunk
 
     if (P.chain == 1) grid_dep_launch();
     for (int i = threadIdx.x; i < TWL; i += blockDim.x) tw[i] = P.tw_row[i];
@@ -413,9 +452,8 @@ __global__ void __launch_bounds__(128, (N >= 1024) ? 2 : (N >= 512 ? 3 : 4)) k_s
             float2 v[PER];
             to_complex(raw, v);
             if (LG == 0) {
-                float *const rowL = rbL + s * N;
 #pragma unroll
-                for (int m = 0; m < PER; m++) rowL[lane + T * m] = hypotf(v[m].x, v[m].y);
+                for (int m = 0; m < PER; m++) ar[s][m] = hypotf(v[m].x, v[m].y);
                 return;
             }
 #pragma unroll
@@ -458,7 +496,8 @@ __global__ void __launch_bounds__(128, (N >= 1024) ? 2 : (N >= 512 ? 3 : 4)) k_s
 
         uint32_t raw[PER];
         load_row(tm, raw);
-#pragma unroll 1
+        constexpr int UNR = (LG == 0) ? RPT : 1;
+#pragma unroll UNR
         for (int ir = 0; ir < RPT; ir++) {
             uint32_t cur[PER];
 #pragma unroll
@@ -471,13 +510,13 @@ __global__ void __launch_bounds__(128, (N >= 1024) ? 2 : (N >= 512 ? 3 : 4)) k_s
         // chunk), extremes, and the FFT input: two real rows in one complex
         // sequence; the slave's rows carry its mask columns [N/4, 3N/4) only
         float *ag = P.rc_amp + (size_t)c * RPC * N;
-        float *acc1 = acc + tm * (N + GOFF);
         float2 v[PER];
+        float sums[PER];
 #pragma unroll
         for (int m = 0; m < PER; m++) {
             const int e = lane + T * m;
-            const float a0 = rbL[e];
-            const float a1 = (RPT == 2) ? rbL[N + e] : 0.f;
+            const float a0 = (LG == 0) ? ar[0][m] : rbL[e];
+            const float a1 = (RPT == 1) ? 0.f : (LG == 0) ? ar[(LG == 0) ? RPT - 1 : 0][m] : rbL[N + e];
             const bool cin = (m >= PER / 4) && (m < 3 * PER / 4);
             const bool use = (img == 0) || cin;
             // the slave's amplitudes are read only inside its mask columns
@@ -486,33 +525,37 @@ __global__ void __launch_bounds__(128, (N >= 1024) ? 2 : (N >= 512 ? 3 : 4)) k_s
                 ag[(size_t)tm * N + e] = a0;
                 if (RPT == 2) ag[(size_t)(TPW + tm) * N + e] = a1;
             }
-            acc1[e] = (RPT == 2) ? a0 + a1 : a0;
+            sums[m] = (RPT == 2) ? a0 + a1 : a0;
             if (use) {
                 mn = fminf(mn, a0); mx = fmaxf(mx, a0);
                 if (RPT == 2) { mn = fminf(mn, a1); mx = fmaxf(mx, a1); }
             }
             v[m] = use ? make_float2(a0, a1) : make_float2(0.f, 0.f);
         }
+        {
+            const float x = chunk_tree<T>(sums, l32);    // the remaining tree levels
+            if (l32 == 0) P.rc_part[c] = x;
+        }
         team_fft_reg<N, -1>(v, ex, tw, lane);
         // half spectra k in [0, N/2) of both rows; bin 0 carries (DC, Nyquist),
-        // both real for a real row
-#pragma unroll
-        for (int m = 0; m < PER; m++) ex[fft_pad(lane + T * m)] = v[m];
-        __syncwarp();
+        // both real for a real row.  Element N - k of k = lane + T m is in lane
+        // T - lane's register PER - 1 - m (lane 0: in its own PER - m)
         float2 *s0 = P.rc_spec + ((size_t)c * RPC + tm) * NH;
         float2 *s1 = P.rc_spec + ((size_t)c * RPC + TPW + tm) * NH;
-        const float2 xn = ex[fft_pad(N / 2)];
+        const int mir = (l32 - lane) + ((T - lane) & (T - 1));
+        const float2 xn = v[PER / 2];                    // k = 0's lane: the Nyquist bin
 #pragma unroll
         for (int m = 0; m < PER / 2; m++) {
             const int k = lane + T * m;
             const float2 z1 = v[m];
             if (RPT == 2) {
-                float2 A, B;
+                float2 A, B, z2 = (lane == 0) ? v[(PER - m) % PER] : v[PER - 1 - m];
+                z2.x = __shfl_sync(0xffffffffu, z2.x, mir);
+                z2.y = __shfl_sync(0xffffffffu, z2.y, mir);
                 if (k == 0) {
                     A = make_float2(z1.x, xn.x);
                     B = make_float2(z1.y, xn.y);
                 } else {
-                    const float2 z2 = ex[fft_pad(N - k)];
                     A = make_float2(0.5f * (z1.x + z2.x), 0.5f * (z1.y - z2.y));
                     B = make_float2(0.5f * (z1.y + z2.y), -0.5f * (z1.x - z2.x));
                 }
@@ -522,22 +565,7 @@ __global__ void __launch_bounds__(128, (N >= 1024) ? 2 : (N >= 512 ? 3 : 4)) k_s
                 s0[k] = (k == 0) ? make_float2(z1.x, xn.x) : z1;
             }
         }
-        __syncwarp();
         oob = __ballot_sync(0xffffffffu, oob) != 0u;
-        // remaining tree levels, strides ACC/2 .. 1 (as k_rows)
-        {
-            float a[ACC / 32];
-#pragma unroll
-            for (int qq = 0; qq < ACC / 32; qq++) a[qq] = acc[l32 + 32 * qq + (32 * qq / N) * GOFF];
-#pragma unroll
-            for (int s = ACC / 64; s >= 1; s >>= 1)
-#pragma unroll
-                for (int qq = 0; qq < s; qq++) a[qq] = a[qq] + a[qq + s];
-            float x = a[0];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) x = x + __shfl_xor_sync(0xffffffffu, x, o);
-            if (l32 == 0) P.rc_part[c] = x;
-        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
@@ -547,7 +575,7 @@ __global__ void __launch_bounds__(128, (N >= 1024) ? 2 : (N >= 512 ? 3 : 4)) k_s
             P.rc_minmax[c] = make_float2(mn, mx);
             P.rc_oob[c] = oob ? 1 : 0;
         }
-        __syncwarp();        // acc and rb are reused by the warp's next chunk
+        __syncwarp();        // ex and rb are reused by the warp's next chunk
     }
 }
 
@@ -995,11 +1023,10 @@ static size_t rc_plan_smem_bytes(int nent) {
 template <int N, int LG>
 static size_t segrows_smem() {
     constexpr int T = fft_lanes(N);
-    constexpr int ACC = (N >= 1024) ? 1024 : 512;
     const int teams = 128 / T;
     return segrows_twiddles<N, LG>() * sizeof(float2) +
-           (size_t)teams * (fft_padded_len(N) * sizeof(float2) + (2 * N + 32) * sizeof(float)) +
-           (LG >= 2 ? (size_t)128 * (N / T) * sizeof(float2) : (size_t)(128 / 32) * (ACC + 32) * sizeof(float));
+           (size_t)teams * (fft_padded_len(N) * sizeof(float2) + segrows_rowbuf(N, LG) * sizeof(float)) +
+           (LG >= 2 ? (size_t)128 * (N / T) * sizeof(float2) : 0);
 }
 template <int M, int LANES = fft_lanes(M)>
 static size_t cols_rc_smem() {
@@ -1084,9 +1111,9 @@ void launch_rc_plan(const Plan &P, cudaStream_t s) {
     // one CTA per image unless the host entry wants the chunks listed by row band
     const int ctas = P.rc_nbands > 0 ? 1 : 2, nent = ctas == 1 ? 2 * P.nwin : P.nwin;
     const size_t sm = rc_plan_smem_bytes(nent);
-    if (nent <= 128) k_rc_plan<128, 1><<<ctas, 128, sm, s>>>(P);
-    else if (nent <= 512) k_rc_plan<512, 1><<<ctas, 512, sm, s>>>(P);
-    else k_rc_plan<512, RC_ENTRIES / 512><<<ctas, 512, sm, s>>>(P);
+    if (nent <= 128) launch_chain(P, k_rc_plan<128, 1>, dim3(ctas), 128, sm, s, 1, false);
+    else if (nent <= 512) launch_chain(P, k_rc_plan<512, 1>, dim3(ctas), 512, sm, s, 1, false);
+    else launch_chain(P, k_rc_plan<512, RC_ENTRIES / 512>, dim3(ctas), 512, sm, s, 1, false);
 }
 
 template <int N>

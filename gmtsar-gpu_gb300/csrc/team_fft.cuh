@@ -303,6 +303,10 @@ __host__ __device__ constexpr float sin32(int k) { return cos32(k - 8); }
 // second pass's butterflies j and j + 16, which are what its radix-2 third
 // pass combines, so one exchange remains of two.  The same operations on the
 // same elements, so the same bits.
+// With 32 lanes (N = 512, 1024) the last pass's inputs are in the lanes l and
+// l ^ 16: lane l forms the butterflies l + 32 i, which take every second of
+// both lanes' outputs, so a lane sends half of its values by shuffles, 16 (32)
+// shared-memory wavefronts where storing and loading them took 64 (128).
 template <int N, int DIR, int PASS, bool HS = false, bool ZMID = false, int T = fft_lanes(N)>
 __device__ __forceinline__ void team_fft_reg_pass(float2 *v, float2 *ex, const float2 *tw, int Ns, int lane) {
     constexpr bool WIDE512 = (N == 512 && T == 16);
@@ -365,6 +369,32 @@ __device__ __forceinline__ void team_fft_reg_pass(float2 *v, float2 *ex, const f
                 dft_reg<2, DIR>(p);
                 v[r] = p[0];
                 v[r + 16] = p[1];
+            }
+        } else if constexpr (T == 32 && PASS == NP - 2) {
+            constexpr int RL = fft_radix(N, NP - 1), NL = N / RL;
+            static_assert(R == 16 && NL == 256 && RL == 2 * IT, "last pass over lanes l and l ^ 16");
+            const float2 *tw2 = tw + (R - 1) * Ns;
+            const bool hi = (lane & 16) != 0;
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                float2 p[RL];
+#pragma unroll
+                for (int it = 0; it < IT; it++) {
+                    const float2 even = u[it][2 * i], odd = u[it][2 * i + 1];
+                    float2 y;
+                    y.x = __shfl_xor_sync(0xffffffffu, hi ? even.x : odd.x, 16);
+                    y.y = __shfl_xor_sync(0xffffffffu, hi ? even.y : odd.y, 16);
+                    p[2 * it] = hi ? y : even;
+                    p[2 * it + 1] = hi ? odd : y;
+                }
+#pragma unroll
+                for (int r = 1; r < RL; r++) {
+                    const float2 w = tw2[(r - 1) * NL + lane + 32 * i];
+                    p[r] = DIR < 0 ? cmulf(p[r], w) : cmulf_conj(p[r], w);
+                }
+                dft_reg<RL, DIR>(p);
+#pragma unroll
+                for (int r = 0; r < RL; r++) v[i + 8 * r] = p[r];
             }
         } else if constexpr (PASS == NP - 1) {
             // last pass: element j + Ns*r with j = lane + T*it and Ns = NR -> register it + r*IT
