@@ -110,7 +110,8 @@ __device__ constexpr float kT1 = 0.414213562373095048802f;
 // multiple of a quarter turn, factored as in the tangent (Linzer-Feig)
 // butterfly: b * (c + i s) = f * (b + i r b) with f the larger of |c|, |s|
 // (signed) and |r| <= 1, so the pair costs 2 + 4 fused operations instead of
-// a 4-operation rotation and 4 additions.
+// a 4-operation rotation and 4 additions; the last four as two two-lane ones
+// (with scalar ones 1000 windows of 128 x 128 took 1% longer).
 template <int M16, int DIR>
 __device__ __forceinline__ void tan_butterfly(float2 &a, float2 &b) {
     constexpr int m = ((M16 % 16) + 16) % 16;
@@ -136,12 +137,16 @@ __device__ __forceinline__ void tan_butterfly(float2 &a, float2 &b) {
         u = make_float2(fmaf(r, b.x, -b.y), fmaf(r, b.y, b.x));
     }
     const float2 a0 = a;
-    a = make_float2(fmaf(f, u.x, a0.x), fmaf(f, u.y, a0.y));
-    b = make_float2(fmaf(-f, u.x, a0.x), fmaf(-f, u.y, a0.y));
+    a = ffma2(make_float2(f, f), u, a0);
+    b = ffma2(make_float2(-f, -f), u, a0);
 }
 
-// One butterfly stage of length LEN inside an R-point register DFT.
-template <int R, int LEN, int DIR, int K>
+// One butterfly stage of length LEN inside an R-point register DFT.  PQ: quarter
+// turns by two-lane operations on the swapped pair.  The swap costs moves, the
+// code is shorter: the better choice from 512 points on, where instruction
+// fetches stall the column stage (40,000 patches of 512 x 512: 31.2 -> 30.3 ms),
+// not below (1000 windows of 128 x 128: 386.4 -> 387.9 us).
+template <int R, int LEN, int DIR, int K, bool PQ>
 struct DftStage {
     static __device__ __forceinline__ void run(float2 *t, int i) {
         if constexpr (K < LEN / 2) {
@@ -151,6 +156,10 @@ struct DftStage {
                 const float2 a = t[i + K], b = t[i + K + LEN / 2];
                 t[i + K] = fadd2(a, b);
                 t[i + K + LEN / 2] = ffma2(b, make_float2(-1.f, -1.f), a);
+            } else if constexpr (M16 == 4 && PQ) {
+                const float2 a = t[i + K], b = make_float2(t[i + K + LEN / 2].y, t[i + K + LEN / 2].x);
+                t[i + K] = ffma2(b, make_float2(-DIR, DIR), a);
+                t[i + K + LEN / 2] = ffma2(b, make_float2(DIR, -DIR), a);
             } else if constexpr ((M16 & 3) == 0) {   // quarter turns: exact swaps and signs
                 float2 a = t[i + K];
                 float2 b = rot16<M16, DIR>(t[i + K + LEN / 2]);
@@ -162,27 +171,27 @@ struct DftStage {
                 t[i + K] = a;
                 t[i + K + LEN / 2] = b;
             }
-            DftStage<R, LEN, DIR, K + 1>::run(t, i);
+            DftStage<R, LEN, DIR, K + 1, PQ>::run(t, i);
         }
     }
 };
 
-template <int R, int LEN, int DIR>
+template <int R, int LEN, int DIR, bool PQ>
 __device__ __forceinline__ void dft_level(float2 *t) {
     if constexpr (LEN <= R) {
 #pragma unroll
-        for (int i = 0; i < R; i += LEN) DftStage<R, LEN, DIR, 0>::run(t, i);
-        dft_level<R, LEN * 2, DIR>(t);
+        for (int i = 0; i < R; i += LEN) DftStage<R, LEN, DIR, 0, PQ>::run(t, i);
+        dft_level<R, LEN * 2, DIR, PQ>(t);
     }
 }
 
 // R-point DFT of v (R = 2, 4, 8, 16) in registers, natural order in and out.
-template <int R, int DIR>
+template <int R, int DIR, bool PQ = false>
 __device__ __forceinline__ void dft_reg(float2 *v) {
     float2 t[R];
 #pragma unroll
     for (int i = 0; i < R; i++) t[i] = v[bitrev_c<R>(i)];
-    dft_level<R, 2, DIR>(t);
+    dft_level<R, 2, DIR, PQ>(t);
 #pragma unroll
     for (int i = 0; i < R; i++) v[i] = t[i];
 }
@@ -190,7 +199,7 @@ __device__ __forceinline__ void dft_reg(float2 *v) {
 // 16-point DFT of a sequence that is zero outside elements [4, 12), natural
 // order in and out: the first butterfly level pairs element k with k + 8,
 // one of which is zero, so that level is copies and negations.
-template <int DIR>
+template <int DIR, bool PQ>
 __device__ __forceinline__ void dft16_mid(float2 *v) {
     float2 t[16];
 #pragma unroll
@@ -205,7 +214,7 @@ __device__ __forceinline__ void dft16_mid(float2 *v) {
             t[i + 1] = v[k];
         }
     }
-    dft_level<16, 4, DIR>(t);
+    dft_level<16, 4, DIR, PQ>(t);
 #pragma unroll
     for (int i = 0; i < 16; i++) v[i] = t[i];
 }
@@ -310,6 +319,7 @@ __host__ __device__ constexpr float sin32(int k) { return cos32(k - 8); }
 template <int N, int DIR, int PASS, bool HS = false, bool ZMID = false, int T = fft_lanes(N)>
 __device__ __forceinline__ void team_fft_reg_pass(float2 *v, float2 *ex, const float2 *tw, int Ns, int lane) {
     constexpr bool WIDE512 = (N == 512 && T == 16);
+    constexpr bool PQ = (N >= 512);
     constexpr int NP = fft_npasses(N);
     constexpr int R = fft_radix(N, PASS);
     constexpr int NR = N / R;
@@ -334,8 +344,8 @@ __device__ __forceinline__ void team_fft_reg_pass(float2 *v, float2 *ex, const f
                     u[r] = make_float2(u[r].x * c - u[r].y * s, u[r].x * s + u[r].y * c);
                 }
             }
-            if constexpr (ZMID) dft16_mid<DIR>(u);
-            else dft_reg<R, DIR>(u);
+            if constexpr (ZMID) dft16_mid<DIR, PQ>(u);
+            else dft_reg<R, DIR, PQ>(u);
             const int j = lane + T * it;
 #pragma unroll
             for (int r = 0; r < R; r++) ex[fft_pad(j * R + r)] = u[r];
@@ -358,7 +368,7 @@ __device__ __forceinline__ void team_fft_reg_pass(float2 *v, float2 *ex, const f
         }
         if constexpr (PASS < NP - 1) __syncwarp();
 #pragma unroll
-        for (int it = 0; it < IT; it++) dft_reg<R, DIR>(u[it]);
+        for (int it = 0; it < IT; it++) dft_reg<R, DIR, PQ>(u[it]);
         if constexpr (WIDE512) {
             // butterfly lane + 16 r of the last pass: outputs r of this lane's two
             const float2 *tw2 = tw + (R - 1) * Ns;
@@ -366,7 +376,7 @@ __device__ __forceinline__ void team_fft_reg_pass(float2 *v, float2 *ex, const f
             for (int r = 0; r < 16; r++) {
                 const float2 w = tw2[lane + 16 * r];
                 float2 p[2] = {u[0][r], DIR < 0 ? cmulf(u[1][r], w) : cmulf_conj(u[1][r], w)};
-                dft_reg<2, DIR>(p);
+                dft_reg<2, DIR, PQ>(p);
                 v[r] = p[0];
                 v[r + 16] = p[1];
             }
@@ -392,7 +402,7 @@ __device__ __forceinline__ void team_fft_reg_pass(float2 *v, float2 *ex, const f
                     const float2 w = tw2[(r - 1) * NL + lane + 32 * i];
                     p[r] = DIR < 0 ? cmulf(p[r], w) : cmulf_conj(p[r], w);
                 }
-                dft_reg<RL, DIR>(p);
+                dft_reg<RL, DIR, PQ>(p);
 #pragma unroll
                 for (int r = 0; r < RL; r++) v[i + 8 * r] = p[r];
             }
