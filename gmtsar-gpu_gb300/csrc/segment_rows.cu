@@ -821,7 +821,10 @@ __global__ void __launch_bounds__(THR, MINB) k_cols_rcp(Plan P) {
     if (t >= tend) return;
     const int warp = threadIdx.x >> 5, l32 = threadIdx.x & 31;
     const int lane = l32 % T;
-    const int team = warp * (32 / T) + l32 / T;
+    // the columns of a warp: all even or all odd, this team's at 4 times tms;
+    // two teams of 8 lanes in a half-warp 8 slots apart, four of 4 lanes 4 slots
+    // apart, which puts them in distinct banks
+    const int tm = l32 / T, tms = (T == 8) ? (tm >> 1) | ((tm & 1) << 1) : tm;
     const int sl = threadIdx.x % CP, row0 = threadIdx.x / CP;   // staging: slot, first row
     // tile t: window t / NG, column group t % NG (a CTA's consecutive tiles
     // are the next column groups of one window; taking the next windows at
@@ -896,9 +899,11 @@ __global__ void __launch_bounds__(THR, MINB) k_cols_rcp(Plan P) {
         }
         cur_w = w;
 
-        const int kx = kx0 + team;
-        float2 *a = cols + team * CS;            // master column, later the result
-        float2 *pa = cols + (CP + team) * CS;    // slave column
+        // even and odd columns differ in work (below), so the warps take turns
+        const int par = (warp ^ t) & 1, slot = par + 2 * (warp >> 1) + 4 * tms;
+        const int kx = kx0 + slot;               // kx0 is even
+        float2 *a = cols + slot * CS;            // master column, later the result
+        float2 *pa = cols + (CP + slot) * CS;    // slave column
         float2 z[PER];
 #pragma unroll
         for (int m = 0; m < PER; m++)
@@ -922,14 +927,26 @@ __global__ void __launch_bounds__(THR, MINB) k_cols_rcp(Plan P) {
         __syncwarp();
         team_fft_reg<M, -1, T>(z, a, tw, lane);
 
+        // The shift's sign (-1)^(kx + ky): the half in ky swaps the halves of the
+        // inverse transform's output, bit for bit (the sign is the same for all
+        // inputs of a butterfly until the pass that adds even and odd inputs, and
+        // swaps its sums and differences), so the stores below swap them instead.
+        // The mask's spectrum is zero in even kx but 0: those columns take no
+        // correction, and in odd ones the sign goes into it (with the warps' columns
+        // of one parity, the column stage of 1000 windows of 128 x 128 187 -> 182
+        // us; of 391 of 128 x 64, also by the banks, 51 -> 43).
         auto product = [&](int kxx, float2 A1, float2 A2, int ky) {
             if (kxx == 0 && ky == 0) A1.x -= dc1;
             const float2 bm = cmulf(boxx[kxx == NH ? CP : kxx - kx0], boxy[ky]);
             A2.x -= m2 * bm.x;
             A2.y -= m2 * bm.y;
             float2 pr = cmulf_conj(A1, A2);
-            if ((kxx + ky) & 1) { pr.x = -pr.x; pr.y = -pr.y; }
+            if (kxx & 1) { pr.x = -pr.x; pr.y = -pr.y; }
             return pr;
+        };
+        auto product_odd = [&](float2 bx, float2 A1, float2 A2, int ky) {
+            const float2 bm = cmulf(bx, boxy[ky]);
+            return cmulf_conj(A1, make_float2(m2 * bm.x - A2.x, m2 * bm.y - A2.y));
         };
         // the product of column kx: from the master spectrum in registers, or
         // in column group 0 (CTA-uniform) through the master slot, where the
@@ -938,12 +955,19 @@ __global__ void __launch_bounds__(THR, MINB) k_cols_rcp(Plan P) {
         const bool dc = (kx == 0);
         const int nout = (b == 0 && __any_sync(0xffffffffu, dc)) ? 2 : 1;    // warp-uniform
         float2 *xs = cols + 2 * CP * CS;
-        if (b != 0) {
+        if (b != 0 && par == 0) {
+#pragma unroll
+            for (int m = 0; m < PER; m++) {
+                if constexpr (KEEP) z[m] = cmulf_conj(z[m], zs[m]);
+                else z[m] = cmulf_conj(z[m], pa[fft_pad(lane + T * m)]);
+            }
+        } else if (b != 0) {
+            const float2 bx = boxx[slot];
 #pragma unroll
             for (int m = 0; m < PER; m++) {
                 const int ky = lane + T * m;
-                if constexpr (KEEP) z[m] = product(kx, z[m], zs[m], ky);
-                else z[m] = product(kx, z[m], pa[fft_pad(ky)], ky);
+                if constexpr (KEEP) z[m] = product_odd(bx, z[m], zs[m], ky);
+                else z[m] = product_odd(bx, z[m], pa[fft_pad(ky)], ky);
             }
         } else {
 #pragma unroll
@@ -983,7 +1007,7 @@ __global__ void __launch_bounds__(THR, MINB) k_cols_rcp(Plan P) {
             __syncwarp();
             team_fft_reg<M, +1, T>(z, dst, tw, lane);
 #pragma unroll
-            for (int m = PER / 4; m < 3 * PER / 4; m++) dst[fft_pad(lane + T * m)] = z[m];
+            for (int m = PER / 4; m < 3 * PER / 4; m++) dst[fft_pad(lane + T * m)] = z[(m + PER / 2) % PER];
             __syncwarp();
         }
         __syncthreads();

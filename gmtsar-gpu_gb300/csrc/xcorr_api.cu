@@ -98,9 +98,15 @@ std::vector<float2> interp_operator(int n, int m) {
 }
 
 // DFT of the 0/1 mask along one axis (make_mask, xcorr.cu:385-401): ones on [lo, n-lo).
+// Half a period of ones (n = 4 lo, every plan's): the even bins but 0 are zero,
+// exactly, which the column stage relies on to skip them.
 std::vector<float2> box_spectrum(int n, int lo) {
     std::vector<float2> b(n);
     for (int k = 0; k < n; k++) {
+        if (n == 4 * lo && k > 0 && k % 2 == 0) {
+            b[k] = make_float2(0.f, 0.f);
+            continue;
+        }
         cd s = 0;
         for (int c = lo; c < n - lo; c++) s += std::polar(1.0, -2.0 * M_PI * (double)k * c / n);
         b[k] = make_float2((float)s.real(), (float)s.imag());
