@@ -404,36 +404,53 @@ __global__ void __launch_bounds__(128, (N >= 1024) ? 2 : (N >= 512 ? 3 : 4)) k_s
     const int cbase = P.nwin * P.nchunks;
     const bool iq16 = (P.format == 0);
 
-    // chunks are taken four per CTA, one per warp; warps share no state
-    // between chunks, so a warp that runs out leaves without a barrier
-    for (int i = begin + 4 * blockIdx.x + warp; i < end; i += 4 * gridDim.x) {
-        const int c = banded ? P.rc_order[i] : (i < cm ? i : cbase + (i - cm));
-        const int4 d = P.rc_desc[c];
-        const int img = d.y;
+    // Chunks are taken four per CTA, one per warp; warps share no state between
+    // chunks, so a warp that runs out leaves without a barrier.  A warp's next
+    // descriptor is read at the start of a chunk and the next chunk's first row
+    // during the current one's last, so neither is waited for (40,000
+    // patches of 512 x 512: 15.6 -> 13.7 ms; 1000 of 256 x 256: 151 -> 140 us).
+    const int step = 4 * gridDim.x;
+    auto chunk_of = [&](int i) { return banded ? P.rc_order[i] : (i < cm ? i : cbase + (i - cm)); };
+    const void *base;
+    int nx, ny, x0, y0, img;
+    auto take = [&](const int4 &d) {
+        img = d.y;
         const PairDev *q = P.pairs ? P.pairs + d.x : nullptr;
-        const void *base = q ? (img ? q->slave : q->master) : (img ? P.single.slave : P.single.master);
-        const int nx = q ? (img ? q->s_nx : q->m_nx) : (img ? P.single.s_nx : P.single.m_nx);
-        const int ny = q ? (img ? q->s_ny : q->m_ny) : (img ? P.single.s_ny : P.single.m_ny);
-        const int x0 = d.z, y0 = d.w;
-        bool oob = false;
+        base = q ? (img ? q->slave : q->master) : (img ? P.single.slave : P.single.master);
+        nx = q ? (img ? q->s_nx : q->m_nx) : (img ? P.single.s_nx : P.single.m_nx);
+        ny = q ? (img ? q->s_ny : q->m_ny) : (img ? P.single.s_ny : P.single.m_ny);
+        x0 = d.z;
+        y0 = d.w;
+    };
+    bool oob = false;                                    // of the chunk whose rows are loaded
+    auto load_row = [&](int r, uint32_t *raw) {
+        const int y = y0 + r;
+        const bool rowok = (y >= 0 && y < ny);
+        const uint32_t *row = reinterpret_cast<const uint32_t *>(base) + (size_t)(rowok ? y : 0) * (size_t)nx;
+        if (rowok && x0 >= 0 && x0 + N <= nx) {
+#pragma unroll
+            for (int m = 0; m < PER; m++) raw[m] = __ldg(row + x0 + lane + T * m);
+        } else {
+#pragma unroll
+            for (int m = 0; m < PER; m++) {
+                const int x = x0 + lane + T * m;
+                if (rowok && x >= 0 && x < nx) raw[m] = __ldg(row + x);
+                else { raw[m] = 0u; oob = true; }
+            }
+        }
+    };
+    int i = begin + 4 * blockIdx.x + warp;
+    if (i >= end) return;
+    int c = chunk_of(i);
+    take(P.rc_desc[c]);
+    uint32_t raw[PER];
+    load_row(tm, raw);
+    for (;;) {
+        const bool more = i + step < end;
+        const int cn = more ? chunk_of(i + step) : c;
+        const int4 dn = P.rc_desc[cn];
         float mn = INFINITY, mx = -INFINITY;
 
-        auto load_row = [&](int r, uint32_t *raw) {
-            const int y = y0 + r;
-            const bool rowok = (y >= 0 && y < ny);
-            const uint32_t *row = reinterpret_cast<const uint32_t *>(base) + (size_t)(rowok ? y : 0) * (size_t)nx;
-            if (rowok && x0 >= 0 && x0 + N <= nx) {
-#pragma unroll
-                for (int m = 0; m < PER; m++) raw[m] = __ldg(row + x0 + lane + T * m);
-            } else {
-#pragma unroll
-                for (int m = 0; m < PER; m++) {
-                    const int x = x0 + lane + T * m;
-                    if (rowok && x >= 0 && x < nx) raw[m] = __ldg(row + x);
-                    else { raw[m] = 0u; oob = true; }
-                }
-            }
-        };
         auto to_complex = [&](const uint32_t *raw, float2 *v) {
             if (iq16) {
 #pragma unroll
@@ -494,15 +511,23 @@ __global__ void __launch_bounds__(128, (N >= 1024) ? 2 : (N >= 512 ? 3 : 4)) k_s
             }
         };
 
-        uint32_t raw[PER];
-        load_row(tm, raw);
+        int cur_img = img;
+        bool any_oob = false;
         constexpr int UNR = (LG == 0) ? RPT : 1;
 #pragma unroll UNR
         for (int ir = 0; ir < RPT; ir++) {
             uint32_t cur[PER];
 #pragma unroll
             for (int m = 0; m < PER; m++) cur[m] = raw[m];
-            if (ir + 1 < RPT) load_row((ir + 1) * TPW + tm, raw);     // in flight during this row
+            // the chunk's next row or the next chunk's first, in flight during this one
+            const bool last = (ir + 1 == RPT);
+            if (last) {
+                cur_img = img;
+                any_oob = __ballot_sync(0xffffffffu, oob) != 0u;
+                oob = false;
+                take(dn);
+            }
+            if (!last || more) load_row(last ? tm : (ir + 1) * TPW + tm, raw);
             amp_row(ir, ir * TPW + tm, cur);
         }
         __syncwarp();
@@ -518,7 +543,7 @@ __global__ void __launch_bounds__(128, (N >= 1024) ? 2 : (N >= 512 ? 3 : 4)) k_s
             const float a0 = (LG == 0) ? ar[0][m] : rbL[e];
             const float a1 = (RPT == 1) ? 0.f : (LG == 0) ? ar[(LG == 0) ? RPT - 1 : 0][m] : rbL[N + e];
             const bool cin = (m >= PER / 4) && (m < 3 * PER / 4);
-            const bool use = (img == 0) || cin;
+            const bool use = (cur_img == 0) || cin;
             // the slave's amplitudes are read only inside its mask columns
             // (the time-correlation window, [xsearch, xsearch + nx_corr))
             if (use) {
@@ -565,7 +590,6 @@ __global__ void __launch_bounds__(128, (N >= 1024) ? 2 : (N >= 512 ? 3 : 4)) k_s
                 s0[k] = (k == 0) ? make_float2(z1.x, xn.x) : z1;
             }
         }
-        oob = __ballot_sync(0xffffffffu, oob) != 0u;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
@@ -573,8 +597,11 @@ __global__ void __launch_bounds__(128, (N >= 1024) ? 2 : (N >= 512 ? 3 : 4)) k_s
         }
         if (l32 == 0) {
             P.rc_minmax[c] = make_float2(mn, mx);
-            P.rc_oob[c] = oob ? 1 : 0;
+            P.rc_oob[c] = any_oob ? 1 : 0;
         }
+        if (!more) break;
+        i += step;
+        c = cn;
         __syncwarp();        // ex and rb are reused by the warp's next chunk
     }
 }
@@ -1144,14 +1171,17 @@ template <int N>
 static void launch_segrows_t(const Plan &P, cudaStream_t s) {
     // a grid-stride walk over the planned chunks, four per CTA; the grid is
     // sized for the chunks the batch would have without sharing, capped at
-    // the CTAs that fit the GPU at once several times over
+    // a multiple of the CTAs that fit the GPU at once: four (a warp reads ahead
+    // from its second chunk on; with an earlier form of it 1000 windows of 128 x 128
+    // took 387 us at eight, 381 at four, 379 at two, where 40,000 of 256 x 256 took
+    // 52.6 ms, 52.5, 52.6), one for a row band, a share of the chunks (1000
+    // windows through host buffers: 547 us, at a half 568, at two 559)
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const size_t maxq = (rc_max_chunks(P.npx, P.npy, P.nwin) + 3) / 4;
     const int per_sm = (N >= 1024) ? 2 : (N >= 512 ? 3 : 4);
-    // a band's launch takes a share of the chunks: a smaller grid
-    const size_t cap = (size_t)sms * per_sm * (P.rc_nbands > 0 ? 2 : 8);
+    const size_t cap = (size_t)sms * per_sm * (P.rc_nbands > 0 ? 1 : 4);
     const int grid = (int)((maxq < cap) ? maxq : cap);
     switch (P.log2ri) {
         case 0: launch_chain(P, k_segrows<N, 0>, dim3(grid), 128, segrows_smem<N, 0>(), s); break;
