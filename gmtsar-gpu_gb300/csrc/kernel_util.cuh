@@ -81,11 +81,12 @@ __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol
 // so a kernel of another split could not start beside the one before it (the
 // strip: 51.8 -> 48.4 us).  With several batches the same split would mix their
 // row and column kernels on an SM, which costs (40,000 windows of 256 x 256:
-// 54.8 -> 61.8 ms), so they keep the splits of their own sizes.
+// 54.8 -> 61.8 ms), so they keep the splits of their own sizes.  3, a lone batch's
+// row bands, which wait for their copies: plain launches with that split.
 template <class Kernel>
 inline void launch_chain(const Plan &P, Kernel kern, dim3 grid, int threads, size_t smem, cudaStream_t s, int cluster = 1,
                          bool dependent = true) {
-    if (!P.chain && cluster == 1) {
+    if (P.chain == 0 && cluster == 1) {
         kern<<<grid, threads, smem, s>>>(P);
         return;
     }
@@ -96,11 +97,11 @@ inline void launch_chain(const Plan &P, Kernel kern, dim3 grid, int threads, siz
     cfg.stream = s;
     cudaLaunchAttribute at[3];
     cfg.attrs = at;
-    if (P.chain == 1) {
+    if (P.chain & 1) {
         at[cfg.numAttrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
         at[cfg.numAttrs++].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
     }
-    if (P.chain && dependent) {
+    if ((P.chain == 1 || P.chain == 2) && dependent) {
         at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
     }

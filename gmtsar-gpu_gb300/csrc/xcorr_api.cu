@@ -824,7 +824,7 @@ xcg_status xcg_correlate(xcg_ctx *c, const void *master, int32_t m_nx, int32_t m
             int lo[2], hi[2];
             for (int k = 0; k < 2; k++) rows_of(Q.win0, Q.win0 + Q.nwin, k, lo[k], hi[k]);
             xcg::Plan Qb = Q;
-            Qb.chain = 0;                 // a band's rows wait for its copy, not only for the launch before
+            Qb.chain = (Q.chain == 1) ? 3 : 0;      // a band's rows wait for its copy, not only for the launch before
             const int nb = std::max(1, std::min(8, Q.nwin / 128));
             Qb.rc_nbands = nb;
             for (int b = 0; b < nb; b++)
