@@ -351,7 +351,10 @@ __device__ __forceinline__ float chunk_tree(float (&t)[PER], int l32) {
 // two.  Range interpolation and amplitudes are k_rows' (xcorr.cu:237-250,
 // fft_interpolate_routines.cu:76-113, conv_ampl_demean.cu:98-108), the chunk
 // sum is h_reduceFD_strip's block sum (conv_ampl_demean.cu:703-726).
-template <int N, int LG>
+// SPEC: the row spectra too; the -time and -time4 modes need none.  (One kernel
+// with a branch took fewer registers, and then its CTAs shared an SM with the peak
+// stage's: 40,000 windows of 256 x 256 52.3 -> 53.0 ms.)
+template <int N, int LG, bool SPEC>
 __global__ void __launch_bounds__(128, (N >= 1024) ? 2 : (N >= 512 ? 3 : 4)) k_segrows(Plan P) {
     constexpr int T = fft_lanes(N);
     constexpr int TPW = 32 / T;
@@ -561,33 +564,35 @@ __global__ void __launch_bounds__(128, (N >= 1024) ? 2 : (N >= 512 ? 3 : 4)) k_s
             const float x = chunk_tree<T>(sums, l32);    // the remaining tree levels
             if (l32 == 0) P.rc_part[c] = x;
         }
-        team_fft_reg<N, -1>(v, ex, tw, lane);
-        // half spectra k in [0, N/2) of both rows; bin 0 carries (DC, Nyquist),
-        // both real for a real row.  Element N - k of k = lane + T m is in lane
-        // T - lane's register PER - 1 - m (lane 0: in its own PER - m)
-        float2 *s0 = P.rc_spec + ((size_t)c * RPC + tm) * NH;
-        float2 *s1 = P.rc_spec + ((size_t)c * RPC + TPW + tm) * NH;
-        const int mir = (l32 - lane) + ((T - lane) & (T - 1));
-        const float2 xn = v[PER / 2];                    // k = 0's lane: the Nyquist bin
+        if constexpr (SPEC) {
+            team_fft_reg<N, -1>(v, ex, tw, lane);
+            // half spectra k in [0, N/2) of both rows; bin 0 carries (DC, Nyquist),
+            // both real for a real row.  Element N - k of k = lane + T m is in lane
+            // T - lane's register PER - 1 - m (lane 0: in its own PER - m)
+            float2 *s0 = P.rc_spec + ((size_t)c * RPC + tm) * NH;
+            float2 *s1 = P.rc_spec + ((size_t)c * RPC + TPW + tm) * NH;
+            const int mir = (l32 - lane) + ((T - lane) & (T - 1));
+            const float2 xn = v[PER / 2];                    // k = 0's lane: the Nyquist bin
 #pragma unroll
-        for (int m = 0; m < PER / 2; m++) {
-            const int k = lane + T * m;
-            const float2 z1 = v[m];
-            if (RPT == 2) {
-                float2 A, B, z2 = (lane == 0) ? v[(PER - m) % PER] : v[PER - 1 - m];
-                z2.x = __shfl_sync(0xffffffffu, z2.x, mir);
-                z2.y = __shfl_sync(0xffffffffu, z2.y, mir);
-                if (k == 0) {
-                    A = make_float2(z1.x, xn.x);
-                    B = make_float2(z1.y, xn.y);
+            for (int m = 0; m < PER / 2; m++) {
+                const int k = lane + T * m;
+                const float2 z1 = v[m];
+                if (RPT == 2) {
+                    float2 A, B, z2 = (lane == 0) ? v[(PER - m) % PER] : v[PER - 1 - m];
+                    z2.x = __shfl_sync(0xffffffffu, z2.x, mir);
+                    z2.y = __shfl_sync(0xffffffffu, z2.y, mir);
+                    if (k == 0) {
+                        A = make_float2(z1.x, xn.x);
+                        B = make_float2(z1.y, xn.y);
+                    } else {
+                        A = make_float2(0.5f * (z1.x + z2.x), 0.5f * (z1.y - z2.y));
+                        B = make_float2(0.5f * (z1.y + z2.y), -0.5f * (z1.x - z2.x));
+                    }
+                    s0[k] = A;
+                    s1[k] = B;
                 } else {
-                    A = make_float2(0.5f * (z1.x + z2.x), 0.5f * (z1.y - z2.y));
-                    B = make_float2(0.5f * (z1.y + z2.y), -0.5f * (z1.x - z2.x));
+                    s0[k] = (k == 0) ? make_float2(z1.x, xn.x) : z1;
                 }
-                s0[k] = A;
-                s1[k] = B;
-            } else {
-                s0[k] = (k == 0) ? make_float2(z1.x, xn.x) : z1;
             }
         }
 #pragma unroll
@@ -1086,16 +1091,16 @@ static size_t cols_rc_smem() {
            (size_t)(M + G::CP + 1) * sizeof(float2) + 4 * sizeof(double) + 16;
 }
 
-template <int N>
+template <int N, bool SPEC>
 static cudaError_t setup_segrows_t() {
     cudaError_t e = cudaSuccess;
     auto set = [&](auto kern, size_t bytes) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     };
-    set(k_segrows<N, 0>, segrows_smem<N, 0>());
-    set(k_segrows<N, 1>, segrows_smem<N, 1>());
-    set(k_segrows<N, 2>, segrows_smem<N, 2>());
-    set(k_segrows<N, 3>, segrows_smem<N, 3>());
+    set(k_segrows<N, 0, SPEC>, segrows_smem<N, 0>());
+    set(k_segrows<N, 1, SPEC>, segrows_smem<N, 1>());
+    set(k_segrows<N, 2, SPEC>, segrows_smem<N, 2>());
+    set(k_segrows<N, 3, SPEC>, segrows_smem<N, 3>());
     return e;
 }
 // The persistent column stage in a form: WIDE (512 points: 16 lanes per
@@ -1134,12 +1139,13 @@ cudaError_t segrows_setup(const Plan &P) {
     cudaError_t e = cudaFuncSetAttribute(k_rc_plan<512, RC_ENTRIES / 512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)rc_plan_smem_bytes(RC_ENTRIES));
     if (e) return e;
+    const bool spec = (P.corr_mode == 2);           // the time modes have 128 columns or more
     switch (P.npx) {
-        case 64: e = setup_segrows_t<64>(); break;
-        case 128: e = setup_segrows_t<128>(); break;
-        case 256: e = setup_segrows_t<256>(); break;
-        case 512: e = setup_segrows_t<512>(); break;
-        case 1024: e = setup_segrows_t<1024>(); break;
+        case 64: e = setup_segrows_t<64, true>(); break;
+        case 128: e = spec ? setup_segrows_t<128, true>() : setup_segrows_t<128, false>(); break;
+        case 256: e = spec ? setup_segrows_t<256, true>() : setup_segrows_t<256, false>(); break;
+        case 512: e = spec ? setup_segrows_t<512, true>() : setup_segrows_t<512, false>(); break;
+        case 1024: e = spec ? setup_segrows_t<1024, true>() : setup_segrows_t<1024, false>(); break;
         default: return cudaErrorInvalidValue;
     }
     if (e) return e;
@@ -1167,7 +1173,7 @@ void launch_rc_plan(const Plan &P, cudaStream_t s) {
     else launch_chain(P, k_rc_plan<512, RC_ENTRIES / 512>, dim3(ctas), 512, sm, s, 1, false);
 }
 
-template <int N>
+template <int N, bool SPEC = true>
 static void launch_segrows_t(const Plan &P, cudaStream_t s) {
     // a grid-stride walk over the planned chunks, four per CTA; the grid is
     // sized for the chunks the batch would have without sharing, capped at
@@ -1184,13 +1190,22 @@ static void launch_segrows_t(const Plan &P, cudaStream_t s) {
     const size_t cap = (size_t)sms * per_sm * (P.rc_nbands > 0 ? 1 : 4);
     const int grid = (int)((maxq < cap) ? maxq : cap);
     switch (P.log2ri) {
-        case 0: launch_chain(P, k_segrows<N, 0>, dim3(grid), 128, segrows_smem<N, 0>(), s); break;
-        case 1: launch_chain(P, k_segrows<N, 1>, dim3(grid), 128, segrows_smem<N, 1>(), s); break;
-        case 2: launch_chain(P, k_segrows<N, 2>, dim3(grid), 128, segrows_smem<N, 2>(), s); break;
-        default: launch_chain(P, k_segrows<N, 3>, dim3(grid), 128, segrows_smem<N, 3>(), s); break;
+        case 0: launch_chain(P, k_segrows<N, 0, SPEC>, dim3(grid), 128, segrows_smem<N, 0>(), s); break;
+        case 1: launch_chain(P, k_segrows<N, 1, SPEC>, dim3(grid), 128, segrows_smem<N, 1>(), s); break;
+        case 2: launch_chain(P, k_segrows<N, 2, SPEC>, dim3(grid), 128, segrows_smem<N, 2>(), s); break;
+        default: launch_chain(P, k_segrows<N, 3, SPEC>, dim3(grid), 128, segrows_smem<N, 3>(), s); break;
     }
 }
 void launch_segrows(const Plan &P, cudaStream_t s) {
+    if (P.corr_mode < 2) {
+        switch (P.npx) {
+            case 128: launch_segrows_t<128, false>(P, s); break;
+            case 256: launch_segrows_t<256, false>(P, s); break;
+            case 512: launch_segrows_t<512, false>(P, s); break;
+            case 1024: launch_segrows_t<1024, false>(P, s); break;
+        }
+        return;
+    }
     switch (P.npx) {
         case 64: launch_segrows_t<64>(P, s); break;
         case 128: launch_segrows_t<128>(P, s); break;

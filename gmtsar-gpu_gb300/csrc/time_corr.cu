@@ -46,8 +46,23 @@ struct TimePlan {
     long long d2;          // sum of b*b (time4: of v*v, modulo 2^64)
     int limbs, shift, rows, pad;
 };
+// A window's amplitudes: the master patch (rows of npx) and the slave's centre
+// (row stride a2s), its own or rows of its chunks of shared row segments
+struct TimeAmps {
+    const float *a1, *a2;
+    int a2s;
+};
+__device__ __forceinline__ TimeAmps time_amps(const Plan &P, int w) {
+    if (P.rc) {
+        const int2 wc = P.rc_wch[w];
+        return {P.rc_amp + (size_t)wc.x * P.rpc * P.npx,
+                P.rc_amp + ((size_t)wc.y * P.rpc + P.ysearch) * P.npx + P.xsearch, P.npx};
+    }
+    return {P.amp1 + (size_t)w * P.npy * P.npx, P.amp2c + (size_t)w * P.ny_corr * P.nx_corr, P.nx_corr};
+}
+
 // A window's arrays in the row-spectrum scratch (npx*npy*8 bytes per window,
-// unused in these modes): cross sums and master energies [nyc][nxc], the plan.
+// P.zrow; with shared row segments the chunks' spectra, both unused in these modes): cross sums and master energies [nyc][nxc], the plan.
 __device__ __forceinline__ char *time_base(const Plan &P, int w) {
     return reinterpret_cast<char *>(P.zrow + (size_t)w * P.npy * P.npx);
 }
@@ -227,14 +242,29 @@ __global__ void __launch_bounds__(TC_THREADS) k_tprep(Plan P, TcGeomArgs G) {
     for (int i = tid; i < 4 * 128; i += TC_THREADS) (&ga[0][0])[i] = 0.f;
     for (int i = tid; i < 4 * 64; i += TC_THREADS) (&gb[0][0])[i] = 0.f;
     if (warp == 0) {   // patch means, as the frequency path forms them, and the digits for the extremes
-        const float *pb = P.part + (size_t)w * 2 * P.nchunks, *mm = P.minmax + (size_t)w * 4 * P.nchunks;
         double s1 = 0.0, s2 = 0.0;
         float lo1 = INFINITY, hi1 = -INFINITY, lo2 = INFINITY, hi2 = -INFINITY;
-        for (int i = l32; i < P.nchunks; i += 32) {
-            s1 += (double)pb[i];
-            s2 += (double)pb[P.nchunks + i];
-            lo1 = fminf(lo1, mm[i]); hi1 = fmaxf(hi1, mm[P.nchunks + i]);
-            lo2 = fminf(lo2, mm[2 * P.nchunks + i]); hi2 = fmaxf(hi2, mm[3 * P.nchunks + i]);
+        if (P.rc) {         // the slave's extremes over its mask rows, as k_peak takes them
+            const int2 wc = P.rc_wch[w];
+            for (int i = l32; i < P.nchunks; i += 32) {
+                s1 += (double)P.rc_part[wc.x + i];
+                s2 += (double)P.rc_part[wc.y + i];
+                const float2 a = P.rc_minmax[wc.x + i];
+                lo1 = fminf(lo1, a.x); hi1 = fmaxf(hi1, a.y);
+                const int r0 = i * P.rpc;
+                if (r0 >= P.ysearch && r0 < P.npy - P.ysearch) {
+                    const float2 b = P.rc_minmax[wc.y + i];
+                    lo2 = fminf(lo2, b.x); hi2 = fmaxf(hi2, b.y);
+                }
+            }
+        } else {
+            const float *pb = P.part + (size_t)w * 2 * P.nchunks, *mm = P.minmax + (size_t)w * 4 * P.nchunks;
+            for (int i = l32; i < P.nchunks; i += 32) {
+                s1 += (double)pb[i];
+                s2 += (double)pb[P.nchunks + i];
+                lo1 = fminf(lo1, mm[i]); hi1 = fmaxf(hi1, mm[P.nchunks + i]);
+                lo2 = fminf(lo2, mm[2 * P.nchunks + i]); hi2 = fmaxf(hi2, mm[3 * P.nchunks + i]);
+            }
         }
         s1 = warp_sum_d(s1);
         s2 = warp_sum_d(s2);
@@ -255,8 +285,8 @@ __global__ void __launch_bounds__(TC_THREADS) k_tprep(Plan P, TcGeomArgs G) {
     }
     __syncthreads();
     const float m1f = (float)mean_sh[0], m2f = (float)mean_sh[1];
-    const float *amp1 = P.amp1 + (size_t)w * P.npy * N;
-    const float *amp2 = P.amp2c + (size_t)w * ny * nx;
+    const TimeAmps amps = time_amps(P, w);
+    const float *amp1 = amps.a1, *amp2 = amps.a2;
     const int L = plan_sh.limbs, sh = plan_sh.shift;
     // adds this thread's digit energies of one group of rows to the group's
     auto publish = [&](float *e, float (*g)[128], float (*g2)[64], int at) {
@@ -279,11 +309,13 @@ __global__ void __launch_bounds__(TC_THREADS) k_tprep(Plan P, TcGeomArgs G) {
     unsigned long long d2 = 0;
     for (int g = warp; g < ny / 8; g += 8) {           // the slave's window: a warp per eight rows
         float e[LMAX] = {};
-        for (int c = l32; c < 8 * nx; c += 32) {
-            const float av = amp2[(size_t)g * 8 * nx + c];
-            const typename Tr::E v = Tr::elem(demeaned_int(av, m2f));
-            d2 += (unsigned long long)Tr::prod(v, v);
-            if (L) add_energy(av, m2f, e);
+        for (int q = 0; q < 8; q++) {
+            const float *row = amp2 + (size_t)(g * 8 + q) * amps.a2s;
+            for (int c = l32; c < nx; c += 32) {
+                const typename Tr::E v = Tr::elem(demeaned_int(row[c], m2f));
+                d2 += (unsigned long long)Tr::prod(v, v);
+                if (L) add_energy(row[c], m2f, e);
+            }
         }
         publish(e, nullptr, gb, g);
     }
@@ -503,8 +535,8 @@ __global__ void __launch_bounds__(256, 1) k_tcorr_tc(Plan P, int KS) {
     volatile int *abort_sh = reinterpret_cast<volatile int *>(tmem_sh + 1);
     volatile int *go = abort_sh + 1;                                       // [2] by the parity of the row step
     const float m1f = (float)P.means[2 * w], m2f = (float)P.means[2 * w + 1];
-    const float *amp1 = P.amp1 + ((size_t)w * P.npy + i0) * N + j0;
-    const float *amp2 = P.amp2c + (size_t)w * ny * nx;
+    const TimeAmps amps = time_amps(P, w);
+    const float *amp1 = amps.a1 + (size_t)i0 * N + j0;
     long long *num = time_num(P, w) + (size_t)i0 * nxc + j0;
     uint32_t tcols = 32;
     while (tcols < (uint32_t)((2 * L - 1) * JT)) tcols <<= 1;
@@ -544,7 +576,7 @@ __global__ void __launch_bounds__(256, 1) k_tcorr_tc(Plan P, int KS) {
 #pragma unroll
                 for (int e = 0; e < 4; e++) pk[l][e] = 0u;
             if (p >= 0 && p < ny) {
-                const float4 *src = reinterpret_cast<const float4 *>(amp2 + (size_t)(ny - 1 - p) * nx + x0 + 8 * kb);
+                const float4 *src = reinterpret_cast<const float4 *>(amps.a2 + (size_t)(ny - 1 - p) * amps.a2s + x0 + 8 * kb);
                 const float4 u = __ldg(src), v = __ldg(src + 1);
                 const float f[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -767,8 +799,9 @@ __global__ void __launch_bounds__(TC_THREADS) k_tcorr(Plan P) {
         if (time_plan(P, w)->limbs != 0) continue;                      // formed on the tensor cores
         const int i0 = (t0 / tiles_j) * TI, j0 = (t0 % tiles_j) * TJ;    // first lag row and column of the tile
         const float m1f = (float)P.means[2 * w], m2f = (float)P.means[2 * w + 1];
-        const float *amp1 = P.amp1 + (size_t)w * P.npy * N;
-        const float *amp2 = P.amp2c + (size_t)w * ny_corr * nx_corr;
+        const TimeAmps amps = time_amps(P, w);
+        const float *amp1 = amps.a1;
+        const int lgx = 31 - __clz(nx_corr);                             // a power of two
         S sab[RI][RJ];
 #pragma unroll
         for (int a = 0; a < RI; a++)
@@ -782,7 +815,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_tcorr(Plan P) {
                 As[t] = Tr::elem(demeaned_int(amp1[(size_t)(y0 + i0 + r) * N + j0 + cc], m1f));
             }
             for (int t = threadIdx.x; t < YB * nx_corr; t += TC_THREADS)
-                Bs[t] = Tr::elem(demeaned_int(amp2[(size_t)y0 * nx_corr + t], m2f));
+                Bs[t] = Tr::elem(demeaned_int(amps.a2[(size_t)(y0 + (t >> lgx)) * amps.a2s + (t & (nx_corr - 1))], m2f));
             __syncthreads();
 #pragma unroll 1
             for (int yy = 0; yy < YB; yy++) {
@@ -877,7 +910,9 @@ __global__ void __launch_bounds__(TC_THREADS) k_tpeak(Plan P) {
     if (l32 == 0) rf[warp] = top;
     if (warp == 0) {          // any chunk that read outside an image, reduced by one warp
         int f = 0;
-        for (int i = l32; i < P.nchunks; i += 32) f |= P.oobmap[(size_t)w * P.nchunks + i];
+        const int2 wc = P.rc ? P.rc_wch[w] : make_int2(0, 0);
+        for (int i = l32; i < P.nchunks; i += 32)
+            f |= P.rc ? P.rc_oob[wc.x + i] | P.rc_oob[wc.y + i] : P.oobmap[(size_t)w * P.nchunks + i];
         f = __any_sync(0xffffffffu, f != 0);
         if (l32 == 0) oob_sh = f;
     }

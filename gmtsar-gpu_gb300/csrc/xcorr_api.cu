@@ -227,7 +227,7 @@ xcg_status xcg_create(const xcg_params *p, int32_t device, int32_t max_batch, xc
     B.nchunks = B.npx * B.npy / 1024;
     B.qpitch = B.npx / 2 + 16;
     B.rpc = B.npx >= 1024 ? 1 : 1024 / B.npx;
-    B.rc = (B.corr_mode == 2) ? 1 : 0;      // the frequency-domain mode shares row segments by default
+    B.rc = 1;                               // row segments are shared by default
 
     // tables
     std::vector<float2> tw_row = stockham_twiddles(B.npx), tw_col = stockham_twiddles(B.npy);
@@ -378,7 +378,7 @@ xcg_status xcg_set_batches(xcg_ctx *c, int32_t batches) {
 
 xcg_status xcg_set_row_sharing(xcg_ctx *c, int32_t enable) {
     if (!c) return XCG_ERR_ARG;
-    c->base.rc = (enable && c->base.corr_mode == 2) ? 1 : 0;
+    c->base.rc = enable ? 1 : 0;
     return XCG_OK;
 }
 
@@ -486,6 +486,16 @@ Plan rows_subrange(Plan P, int off, int n) {
     return P;
 }
 
+// Whether a job of nlocs windows runs on shared row segments.  In the -time and
+// -time4 modes from 2^24 pixels of patches on: the row stage per window takes 5 to 7
+// us per million, and sharing has a planner to pay (17 us) however little the
+// windows overlap (1000 windows of 128 x 128: 3037 -> 2828 us; 400 of 64 x 64, 6.5
+// million pixels that barely overlap: 536 -> 550).
+static bool shares_rows(const Plan &P, int nlocs) {
+    if (!P.rc || P.tc_form) return false;             // the precision form reads the per-window arrays
+    return P.corr_mode == 2 || (size_t)nlocs * P.npx * P.npy >= ((size_t)1 << 24);
+}
+
 int ctx_batch_windows(const xcg_ctx *c, int nlocs, int strip_len) {
     // With one row stage per window, as many windows per batch as the scratch
     // holds: one 1000-window launch per stage fills the GPU better than two
@@ -495,12 +505,13 @@ int ctx_batch_windows(const xcg_ctx *c, int nlocs, int strip_len) {
     // one-CTA-per-SM tensor stages: 626 K against 601 K windows/s) and on
     // shared row segments (the second batch's row stage overlaps the first's
     // column stage: 0.548 against 0.563 ms per 1000 windows of 128x128, and
-    // in the host entry its image copy too: 0.732 against 0.791 ms).  On the
+    // in the host entry its image copy too: 0.732 against 0.791 ms; -time 2749
+    // against 2828 us).  On the
     // host entry a first batch of a quarter of the windows measured the same
     // as two halves (0.702 against 0.703 ms per call): the call's timeline
     // shows the device busy from the end of the first batch's row stage on.
     int bw = c->max_batch;
-    if ((c->base.tc_form || c->base.rc) && nlocs >= 512 && (nlocs + 1) / 2 < bw) bw = (nlocs + 1) / 2;
+    if ((c->base.tc_form || shares_rows(c->base, nlocs)) && nlocs >= 512 && (nlocs + 1) / 2 < bw) bw = (nlocs + 1) / 2;
     if (c->batches_cfg > 0) bw = std::min(c->max_batch, (nlocs + c->batches_cfg - 1) / c->batches_cfg);
     if (strip_len > 0 && strip_len <= bw) bw = ((bw + strip_len - 1) / strip_len) * strip_len;   // whole strips
     if (bw > c->max_batch) bw = (c->max_batch / (strip_len > 0 ? strip_len : 1)) * (strip_len > 0 ? strip_len : 1);
@@ -513,9 +524,7 @@ xcg_status ctx_launch(xcg_ctx *c, Plan P, const int *starts, int nb, cudaStream_
     // launch slots: rows, columns, peak, subpixel; the precision form splits
     // the column stage into three tensor-core DFT stages
     const bool tcf = P.tc_form != 0;
-    // shared row segments: frequency-domain FP32 path only (the precision
-    // form and the time modes read the per-window arrays)
-    if (tcf || P.corr_mode < 2) P.rc = 0;
+    P.rc = shares_rows(P, starts[nb] - starts[0]) ? 1 : 0;
     const bool rc = P.rc != 0;
     const int nk = (tcf ? 6 : 4) - (P.interp_flag ? 0 : 1);
     if (c->profiling == 1) {
@@ -551,7 +560,7 @@ xcg_status ctx_launch(xcg_ctx *c, Plan P, const int *starts, int nb, cudaStream_
     // profiling, whose events lie between them, nor into a captured graph,
     // which keeps plain kernel edges)
     P.chain = 0;
-    if (rc && c->profiling == 0 && P.cols_cfg != 1) {
+    if (rc && P.corr_mode == 2 && c->profiling == 0 && P.cols_cfg != 1) {
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
         if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) P.chain = nb == 1 ? 1 : 2;
     }
@@ -586,6 +595,7 @@ xcg_status ctx_launch(xcg_ctx *c, Plan P, const int *starts, int nb, cudaStream_
         if (Q.nwin > maxw) maxw = Q.nwin;
         Q.locs = locs0 + Q.win0;
         Q.winref = ref0 ? ref0 + Q.win0 : nullptr;
+        if (rc && Q.corr_mode < 2) Q.zrow = Q.rc_spec;     // the time modes' sums, where the chunks' spectra would be
         for (int k = 0; k < nk; k++) {
             if (c->profiling == 1) cudaEventRecord(c->events[ei++], ss);
             const bool tm = Q.corr_mode < 2;     // -time / -time4: full-search surface

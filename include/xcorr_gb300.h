@@ -231,8 +231,8 @@ void xcg_stack_get_stats(const xcg_stack *st, xcg_stack_stats *out);
  * its rows; 0 computes them once per window, as the reference's
  * do_correlation does (xcorr.cu:330-338 with d_assign_values, :237-292).
  * Amplitudes, means and the time-domain correlation are the same bits either
- * way; the spectra differ by FP32 rounding.  The precision form and the
- * -time/-time4 modes always run the per-window row stage. */
+ * way (so the -time/-time4 modes' results are too); the spectra differ by FP32
+ * rounding.  The precision form always runs the per-window row stage. */
 xcg_status xcg_set_row_sharing(xcg_ctx *ctx, int32_t enable);
 
 /* Launch shapes of this context's column and peak stages (the choices
