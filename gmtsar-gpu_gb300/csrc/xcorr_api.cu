@@ -510,7 +510,17 @@ int ctx_batch_windows(const xcg_ctx *c, int nlocs, int strip_len) {
     // host entry a first batch of a quarter of the windows measured the same
     // as two halves (0.702 against 0.703 ms per call): the call's timeline
     // shows the device busy from the end of the first batch's row stage on.
+    // Two batches also for 96 to 384 windows with 2^21 pixels of patches or more:
+    // their kernels fill the GPU to a half or less and overlap well (144 windows of
+    // 64 x 64 60 -> 54 us, 192 of 256 x 256 540 -> 457, through host buffers 200 of
+    // 128 x 128 321 -> 269; over 70 grids of this range 0.97 to 1.21, most 1.04 to
+    // 1.14).  Fewer windows lose in the launches and in shared rows (40 of 128 x 128:
+    // 61 against 63 us), smaller ones too (120 of 64 x 64, 1.9 million pixels: 52
+    // against 60); 400 to 511 measured from 0.96 to 1.03.
     int bw = c->max_batch;
+    const size_t px = (size_t)nlocs * c->base.npx * c->base.npy;
+    const bool few = c->base.corr_mode == 2 && c->base.rc && !c->base.tc_form && nlocs >= 96 && nlocs <= 384 && px >= ((size_t)1 << 21);
+    if (few && (nlocs + 1) / 2 < bw) bw = (nlocs + 1) / 2;
     if ((c->base.tc_form || shares_rows(c->base, nlocs)) && nlocs >= 512 && (nlocs + 1) / 2 < bw) bw = (nlocs + 1) / 2;
     if (c->batches_cfg > 0) bw = std::min(c->max_batch, (nlocs + c->batches_cfg - 1) / c->batches_cfg);
     if (strip_len > 0 && strip_len <= bw) bw = ((bw + strip_len - 1) / strip_len) * strip_len;   // whole strips
