@@ -517,11 +517,16 @@ int ctx_batch_windows(const xcg_ctx *c, int nlocs, int strip_len) {
     // 1.14).  Fewer windows lose in the launches and in shared rows (40 of 128 x 128:
     // 61 against 63 us), smaller ones too (120 of 64 x 64, 1.9 million pixels: 52
     // against 60); 400 to 511 measured from 0.96 to 1.03.
+    // Neither these nor the time modes' two batches cut a strip: the last window
+    // before a cut does not see the next one's first value.
     int bw = c->max_batch;
-    const size_t px = (size_t)nlocs * c->base.npx * c->base.npy;
-    const bool few = c->base.corr_mode == 2 && c->base.rc && !c->base.tc_form && nlocs >= 96 && nlocs <= 384 && px >= ((size_t)1 << 21);
-    if (few && (nlocs + 1) / 2 < bw) bw = (nlocs + 1) / 2;
-    if ((c->base.tc_form || shares_rows(c->base, nlocs)) && nlocs >= 512 && (nlocs + 1) / 2 < bw) bw = (nlocs + 1) / 2;
+    const Plan &B = c->base;
+    const int half = (nlocs + 1) / 2;
+    const bool whole = strip_len <= half, freq = B.corr_mode == 2;
+    const bool few = freq && B.rc && !B.tc_form && whole && nlocs >= 96 && nlocs <= 384 &&
+                     (size_t)nlocs * B.npx * B.npy >= ((size_t)1 << 21);
+    const bool many = nlocs >= 512 && (B.tc_form || (shares_rows(B, nlocs) && (freq || whole)));
+    if (few || many) bw = std::min(bw, half);
     if (c->batches_cfg > 0) bw = std::min(c->max_batch, (nlocs + c->batches_cfg - 1) / c->batches_cfg);
     if (strip_len > 0 && strip_len <= bw) bw = ((bw + strip_len - 1) / strip_len) * strip_len;   // whole strips
     if (bw > c->max_batch) bw = (c->max_batch / (strip_len > 0 ? strip_len : 1)) * (strip_len > 0 ? strip_len : 1);
