@@ -505,8 +505,7 @@ int ctx_batch_windows(const xcg_ctx *c, int nlocs, int strip_len) {
     // one-CTA-per-SM tensor stages: 626 K against 601 K windows/s) and on
     // shared row segments (the second batch's row stage overlaps the first's
     // column stage: 0.548 against 0.563 ms per 1000 windows of 128x128, and
-    // in the host entry its image copy too: 0.732 against 0.791 ms; -time 2749
-    // against 2828 us).  On the
+    // in the host entry its image copy too: 0.732 against 0.791 ms).  On the
     // host entry a first batch of a quarter of the windows measured the same
     // as two halves (0.702 against 0.703 ms per call): the call's timeline
     // shows the device busy from the end of the first batch's row stage on.
@@ -525,8 +524,12 @@ int ctx_batch_windows(const xcg_ctx *c, int nlocs, int strip_len) {
     const bool whole = strip_len <= half, freq = B.corr_mode == 2;
     const bool few = freq && B.rc && !B.tc_form && whole && nlocs >= 96 && nlocs <= 384 &&
                      (size_t)nlocs * B.npx * B.npy >= ((size_t)1 << 21);
-    const bool many = nlocs >= 512 && (B.tc_form || (shares_rows(B, nlocs) && (freq || whole)));
-    if (few || many) bw = std::min(bw, half);
+    const bool many = freq && nlocs >= 512 && (B.tc_form || B.rc);
+    // The time modes from 400 windows on (1.01 to 1.10 over ten grids; 200 to 300:
+    // 0.98 to 1.04), -time4 up to 64 x 128 windows (128 x 128 lose: 600 of them 13.7
+    // against 15.2 ms).
+    const bool time = !freq && whole && nlocs >= 400 && (B.corr_mode == 0 || B.nx_corr * B.ny_corr <= 64 * 128);
+    if (few || many || time) bw = std::min(bw, half);
     if (c->batches_cfg > 0) bw = std::min(c->max_batch, (nlocs + c->batches_cfg - 1) / c->batches_cfg);
     if (strip_len > 0 && strip_len <= bw) bw = ((bw + strip_len - 1) / strip_len) * strip_len;   // whole strips
     if (bw > c->max_batch) bw = (c->max_batch / (strip_len > 0 ? strip_len : 1)) * (strip_len > 0 ? strip_len : 1);

@@ -15,7 +15,8 @@ torch = pytest.importorskip("torch")
     (32, 2, 1, 127, 1, 1), (32, 2, 16, 8, 16, 2),            # below, at 2^21 pixels of patches
     (32, 2, 24, 16, 24, 2), (32, 2, 11, 35, 11, 1),          # 384, 385 windows
     (64, 2, 120, 1, 120, 1), (64, 2, 60, 2, 60, 2), (64, 2, 10, 11, 0, 2),      # one strip, two, no strips
-    (64, 0, 17, 15, 17, 1), (64, 0, 32, 16, 32, 2), (64, 0, 8, 64, 512, 1)])    # -time: 255, 512 windows, one strip
+    (64, 0, 21, 19, 21, 1), (64, 0, 20, 20, 20, 2), (32, 1, 20, 20, 20, 2),     # time modes: 399, 400 windows
+    (64, 1, 20, 20, 20, 1), (64, 0, 8, 64, 512, 1)])                            # large -time4 windows, one strip
 def test_split_of_a_job(xs, mode, nxl, nyl, strip, batches):
     n, nx, ny = nxl * nyl, 8 * xs + 3 * nxl + 70, 8 * xs + 3 * nyl + 90
     m, s = synth.make_pair(synth.PairSpec(nx=nx, ny=ny, dx=1.2, dy=-0.7, noise_frac=0.1, seed=n))
