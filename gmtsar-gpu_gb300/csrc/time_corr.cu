@@ -224,6 +224,32 @@ __device__ int rows_per_drain(const float (*ga)[128], const float (*gb)[64], int
     }
 }
 
+// -time4 windows whose energies leave less than eight rows per drain with three
+// digits: four digits and eight rows, if the digits' largest values alone keep
+// every partial sum of 8 nx products below 2^24.  (The integer kernel takes 1.5 ms
+// for such a window however few there are: 60 windows of 128 x 128 2663 -> 1378 us,
+// 600 of them 13.7 -> 8.6 ms.)
+__device__ bool four_digits(TimePlan &t, float vmax, int nx) {
+    for (int s = 7; s <= 8; s++) {
+        const float low = exp2f((float)(s - 1)), top = vmax * vmax * exp2f((float)(-3 * s)) + 2.f;
+        const float d[4] = {low, low, low, top};
+        float worst = 0.f;
+        for (int w = 0; w < 7; w++) {
+            float sum = 0.f;
+            for (int i = 0; i < 4; i++)
+                if (w - i >= 0 && w - i < 4) sum += d[i] * d[w - i];
+            worst = fmaxf(worst, sum);
+        }
+        if (top <= 2048.f && worst * 8.f * (float)nx < 16777216.f * 0.95f) {
+            t.limbs = 4;
+            t.shift = s;
+            t.rows = 8;
+            return true;
+        }
+    }
+    return false;
+}
+
 // CPT: window columns nxc + nx_corr - 1 (below 256 CPT) per thread
 template <int MODE, int CPT>
 __global__ void __launch_bounds__(TC_THREADS) k_tprep(Plan P, TcGeomArgs G) {
@@ -235,6 +261,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_tprep(Plan P, TcGeomArgs G) {
     __shared__ double mean_sh[2];
     __shared__ float ga[4][128], gb[4][64];            // digit energies per eight rows
     __shared__ TimePlan plan_sh;
+    __shared__ float vmax_sh;
     __shared__ unsigned long long red[8];
     const int w = blockIdx.x, tid = threadIdx.x, l32 = tid & 31, warp = tid >> 5;
     const int N = P.npx, nx = P.nx_corr, ny = P.ny_corr, nxc = P.nxc, nyc = P.nyc;
@@ -280,7 +307,8 @@ __global__ void __launch_bounds__(TC_THREADS) k_tprep(Plan P, TcGeomArgs G) {
             mean_sh[0] = s1; mean_sh[1] = s2;
             P.means[2 * w] = s1; P.means[2 * w + 1] = s2;
             const float m1 = (float)s1, m2 = (float)s2;
-            choose_digits<MODE>(plan_sh, fmaxf(fmaxf(hi1 - m1, m1 - lo1), fmaxf(hi2 - m2, m2 - lo2)) * 1.001f + 1.f);
+            vmax_sh = fmaxf(fmaxf(hi1 - m1, m1 - lo1), fmaxf(hi2 - m2, m2 - lo2)) * 1.001f + 1.f;
+            choose_digits<MODE>(plan_sh, vmax_sh);
         }
     }
     __syncthreads();
@@ -403,7 +431,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_tprep(Plan P, TcGeomArgs G) {
         if (l32 == 0) {
             TimePlan t = plan_sh;
             t.rows = rows;
-            if (rows == 0) t.limbs = 0;
+            if (rows == 0 && !(MODE == 1 && L == 3 && four_digits(t, vmax_sh, nx))) t.limbs = 0;
             t.d2 = 0;
             for (int i = 0; i < 8; i++) t.d2 += (long long)red[i];
             *time_plan(P, w) = t;

@@ -526,8 +526,9 @@ int ctx_batch_windows(const xcg_ctx *c, int nlocs, int strip_len) {
                      (size_t)nlocs * B.npx * B.npy >= ((size_t)1 << 21);
     const bool many = freq && nlocs >= 512 && (B.tc_form || B.rc);
     // The time modes from 400 windows on (1.01 to 1.10 over ten grids; 200 to 300:
-    // 0.98 to 1.04), -time4 up to 64 x 128 windows (128 x 128 lose: 600 of them 13.7
-    // against 15.2 ms).
+    // 0.98 to 1.04), -time4 up to 64 x 128 windows (128 x 128 gain nothing, 600 of them
+    // 8.60 against 8.55 ms, and lose where the integer kernel takes windows, 13.7
+    // against 15.2).
     const bool time = !freq && whole && nlocs >= 400 && (B.corr_mode == 0 || B.nx_corr * B.ny_corr <= 64 * 128);
     if (few || many || time) bw = std::min(bw, half);
     if (c->batches_cfg > 0) bw = std::min(c->max_batch, (nlocs + c->batches_cfg - 1) / c->batches_cfg);
