@@ -17,7 +17,8 @@
 //               partial sum an integer below 2^24 and so exact
 //   k_tcorr     the same sums with 64-bit integer multiply-adds, for the
 //               windows whose integers are too large for that (-real images
-//               beyond 2^20; squares beyond 2^31)
+//               beyond 2^20; squares beyond 2^31) or where a wait of k_tcorr_tc
+//               ran out
 //   k_tpeak     per window: the scan-order peak, outputs, 8x8 neighbourhood
 // All sums are 64-bit (time: exact; time4: modulo 2^64 like the reference's
 // long long).
@@ -42,9 +43,13 @@ constexpr int RI = 2, RJ = 4;
 // digits of `shift` bits, the lower ones balanced in [-2^(shift-1),
 // 2^(shift-1)), and the digit products of `rows` master rows accumulate in
 // tensor memory before they are drained; limbs 0: k_tcorr takes the window.
+// k_tcorr_tc only reads these: its CTAs share a window and decide by them which
+// barriers they take.  What it reports goes into `failed`: 0, 1 where one of its
+// waits ran out (k_tcorr forms the window's sums), 2 where its instructions had
+// not ended by the limit of a second wait either (the record says so).
 struct TimePlan {
     long long d2;          // sum of b*b (time4: of v*v, modulo 2^64)
-    int limbs, shift, rows, pad;
+    int limbs, shift, rows, failed;
 };
 // A window's amplitudes: the master patch (rows of npx) and the slave's centre
 // (row stride a2s), its own or rows of its chunks of shared row segments
@@ -162,7 +167,7 @@ __device__ __forceinline__ void digits_of(float amp, float mean, int L, int s, s
 // The top digit must be an integer an f16 holds (2048).  limbs 0: none.
 template <int MODE>
 __device__ void choose_digits(TimePlan &t, float vmax) {
-    t.limbs = t.shift = t.rows = t.pad = 0;
+    t.limbs = t.shift = t.rows = t.failed = 0;
     if (!(vmax >= 0.f) || !(vmax < 1e9f)) return;
     const float top = MODE == 0 ? vmax : vmax * vmax;
     const float lg = log2f(fmaxf(top, 2.f));
@@ -463,6 +468,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_tprep(Plan P, TcGeomArgs G) {
 constexpr int TCT_STAGES = 3;
 constexpr int TCT_PROD = 224;                       // producer threads: warps 1 to 7
 constexpr uint32_t TCT_POLLS = 1u << 18;
+constexpr int TCT_GIVEUP_ROW = 5;                   // Plan::time_giveup: the master row before which a tile gives up
 
 struct TcLayout {
     int rows, hc, rw;                               // A rows, Hankel core matrices, row-buffer halves
@@ -548,7 +554,9 @@ __global__ void __launch_bounds__(256, 1) k_tcorr_tc(Plan P, int KS) {
     // (the shuffles tell the compiler that these are the same for the warp)
     const int L = __shfl_sync(0xffffffffu, plan->limbs, 0), sh = __shfl_sync(0xffffffffu, plan->shift, 0);
     const int seg_rows = __shfl_sync(0xffffffffu, plan->rows, 0);
-    if (L == 0) return;                                       // k_tcorr's window
+    if (L == 0) return;                                       // k_tcorr's window (the same for every warp: nothing here writes limbs)
+    // a test's give-up before this row's wait, with matrix instructions issued already
+    const int giveup = (P.time_giveup && blockIdx.x == 0) ? TCT_GIVEUP_ROW : -1;
     const int nx = P.nx_corr, ny = P.ny_corr, nxc = P.nxc, N = P.npx;
     const int tiles_j = nxc / JT;
     const int i0 = ((int)blockIdx.x / tiles_j) * 128, j0 = ((int)blockIdx.x % tiles_j) * JT;
@@ -634,7 +642,8 @@ __global__ void __launch_bounds__(256, 1) k_tcorr_tc(Plan P, int KS) {
                 const uint32_t hi = (uint32_t)(tc::sdesc(0, 0, 128) >> 32);
                 const uint32_t ad = (uint32_t)(lay.a_limb >> 4), as = 2u * (uint32_t)R, bd = (uint32_t)HC * 8u;
                 const uint32_t sb = (tc::smem_addr(stages) >> 4) | ((JT == 128 ? 8u : 64u * (uint32_t)L) << 16), ss = (uint32_t)(lay.stage >> 4);
-                for (int r = r0; r < r1; r++) {
+                const int rend = (giveup >= r0 && giveup < r1) ? giveup : r1;
+                for (int r = r0; r < rend; r++) {
                     if (!__all_sync(0xffffffffu, !*abort_sh && tc::mbar_wait(&full[st], ph, TCT_POLLS))) {
                         *abort_sh = 1;
                         break;
@@ -656,6 +665,7 @@ __global__ void __launch_bounds__(256, 1) k_tcorr_tc(Plan P, int KS) {
                     alo -= 1u;                                // the next master row: the slave rows one further
                     if (++st == TCT_STAGES) { st = 0; ph ^= 1u; }
                 }
+                if (rend < r1) *abort_sh = 1;
                 if (leader) tc::mma_commit(done);
                 __syncwarp();
             } else {                                          // producers of the Hankel core matrices
@@ -799,8 +809,17 @@ __global__ void __launch_bounds__(256, 1) k_tcorr_tc(Plan P, int KS) {
             for (int e = 0; e < 16; e++) dst[e] = make_ulonglong2(kept[2 * e], kept[2 * e + 1]);
         }
     }
-    if (fail && tid == 0) plan->limbs = 0;                    // a wait ran out: k_tcorr forms this window's sums
+    if (fail) {
+        // a wait ran out: k_tcorr forms this window's sums.  The instructions
+        // committed to `done` may still read shared memory and write tensor
+        // memory, so they end before either is given back
+        const int ended = tc::mbar_wait(done, (seg - 1) & 1, 8 * TCT_POLLS) ? 1 : 0;
+        const bool all = __syncthreads_and(ended) != 0;
+        if (tid == 0) atomicMax(&plan->failed, all ? 1 : 2);
+    }
+    tc::fence_before_sync();
     __syncthreads();
+    tc::fence_after_sync();
     if (warp == 0) tc::tmem_dealloc(tmem, tcols);
 }
 
@@ -824,7 +843,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_tcorr(Plan P) {
 #pragma unroll 1
     for (int item = blockIdx.x; item < P.nwin * tiles; item += gridDim.x) {
         const int w = item / tiles, t0 = item - w * tiles;
-        if (time_plan(P, w)->limbs != 0) continue;                      // formed on the tensor cores
+        if (time_plan(P, w)->limbs != 0 && time_plan(P, w)->failed == 0) continue;      // formed on the tensor cores
         const int i0 = (t0 / tiles_j) * TI, j0 = (t0 % tiles_j) * TJ;    // first lag row and column of the tile
         const float m1f = (float)P.means[2 * w], m2f = (float)P.means[2 * w + 1];
         const TimeAmps amps = time_amps(P, w);
@@ -906,7 +925,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_tpeak(Plan P) {
     __shared__ float rf[8];
     __shared__ double rd[8];
     __shared__ int ri_[8];
-    __shared__ int oob_sh;
+    __shared__ int flags_sh;
     const int w = blockIdx.x;
     const int nxc = P.nxc, nyc = P.nyc, ns = nxc * nyc;
     const long long *num = time_num(P, w), *en = time_energy(P, w);
@@ -936,13 +955,13 @@ __global__ void __launch_bounds__(TC_THREADS) k_tpeak(Plan P) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
     if (l32 == 0) rf[warp] = top;
-    if (warp == 0) {          // any chunk that read outside an image, reduced by one warp
+    if (warp == 0) {          // the record's flags: any chunk that read outside an image, reduced by one warp
         int f = 0;
         const int2 wc = P.rc ? P.rc_wch[w] : make_int2(0, 0);
         for (int i = l32; i < P.nchunks; i += 32)
             f |= P.rc ? P.rc_oob[wc.x + i] | P.rc_oob[wc.y + i] : P.oobmap[(size_t)w * P.nchunks + i];
         f = __any_sync(0xffffffffu, f != 0);
-        if (l32 == 0) oob_sh = f;
+        if (l32 == 0) flags_sh = (f ? XCG_FLAG_OOB : 0) | (time_plan(P, w)->failed > 1 ? XCG_FLAG_STAGE_TIMEOUT : 0);
     }
     __syncthreads();
 #pragma unroll
@@ -991,7 +1010,7 @@ __global__ void __launch_bounds__(TC_THREADS) k_tpeak(Plan P) {
         o.yoff = -1 * ipeak;
         o.corr = F;
         o.ip = ip; o.jp = jp;
-        o.flags = oob_sh ? XCG_FLAG_OOB : 0;
+        o.flags = flags_sh;
         o.cmax = vstar;
         o.cave = 0.0;
         o.cave_true = 0.0;

@@ -583,6 +583,10 @@ xcg_status ctx_launch(xcg_ctx *c, Plan P, const int *starts, int nb, cudaStream_
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
         if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) P.chain = nb == 1 ? 1 : 2;
     }
+    if (P.corr_mode < 2) {
+        P.time_giveup = c->inject_tc_timeout;
+        c->inject_tc_timeout = 0;
+    }
     if (tcf) {             // a timeout of an earlier call must not be reported by this one
         const xcg_status rs = tc_reset_status(c, s);
         if (rs != XCG_OK) return rs;

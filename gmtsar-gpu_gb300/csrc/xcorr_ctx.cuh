@@ -61,6 +61,7 @@ struct xcg_ctx {
     uint8_t *tc_prep = nullptr;
     int *tc_err = nullptr;
     int inject_tc_timeout = 0;    // xcg_debug_inject_stage_timeout: the next call sets the flag instead of clearing it
+                                  // (the time modes: sets Plan::time_giveup)
     // profiling: 1 events around each launch, 2 timeline marks
     int profiling = 0;
     std::vector<cudaEvent_t> events;

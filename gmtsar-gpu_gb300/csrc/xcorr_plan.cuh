@@ -32,6 +32,7 @@ struct Plan {
     int interp_flag, ifc, n2x, n2y, nx2, ny2;
     int format;            // 0 complex int16, 1 float32 real
     int corr_mode;         // 2 frequency domain; 0 -time, 1 -time4 full search
+    int time_giveup;       // 1: each window's first lag tile gives up, as where a wait runs out (xcg_debug_inject_stage_timeout)
     // precision form: the correlation's row/column DFTs as split-FP16
     // tensor-core matmuls (tc_dft.cu); 0 = FP32 SIMT FFTs
     int tc_form;

@@ -58,7 +58,9 @@ enum { XCG_FLAG_OOB = 1,        /* part of a patch fell outside its image and wa
        XCG_FLAG_NEXTREAD = 2,   /* the 8x8 neighbourhood used the next window's first surface value */
        XCG_FLAG_REFINED = 4,    /* xfrac/yfrac come from the subpixel refiner, not the FFT interpolation */
        XCG_FLAG_STAGE_TIMEOUT = 8 };  /* precision form: a tensor-core stage's bounded wait ran out during this
-                                         call, so this window's surface may be incomplete; the result is not valid */
+                                         call, so this window's surface may be incomplete; the result is not valid.
+                                         -time, -time4: instructions of this window's tensor-core stage had not ended
+                                         after a second wait (the sums are then the integer kernel's) */
 
 /* Per-location result. */
 typedef struct {
@@ -338,8 +340,11 @@ xcg_status xcg_set_dft_form(xcg_ctx *ctx, int32_t form);
  * proceeds as if one of its tensor-core waits had run out (the error flag the
  * stages raise is set on the host side instead of cleared at the start of the
  * call): its windows carry XCG_FLAG_STAGE_TIMEOUT and xcg_correlate returns
- * XCG_ERR_CUDA.  The call after it clears the flag again.  For tests of the
- * error path; nothing on the device times out. */
+ * XCG_ERR_CUDA.  The call after it clears the flag again.  On a -time or -time4
+ * context each window's first lag tile gives up on the tensor cores, as where a
+ * wait runs out, and the window's sums are formed on the integer pipe: the
+ * results are the same.  For tests of the error path; nothing on the device
+ * times out. */
 void xcg_debug_inject_stage_timeout(xcg_ctx *ctx);
 
 /* Diagnostic: the split-FP16 tensor-core GEMM engine of the precision form
