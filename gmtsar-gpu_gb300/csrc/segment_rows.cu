@@ -41,6 +41,7 @@
 #include "kernel_util.cuh"
 #include "segment_rows.cuh"
 #include "team_fft.cuh"
+#include "tile_walk.cuh"
 
 namespace xcg {
 
@@ -839,18 +840,19 @@ __global__ void __launch_bounds__(THR, MINB) k_cols_rcp(Plan P) {
     grid_dep_wait();                 // the row stage's spectra and sums
     const bool dyn = (P.rc_tile_next != nullptr);
     const int K = max(1, min(NG / 4, ntiles / (2 * (int)gridDim.x)));
-    int t, tend;                                // the current chunk [t, tend)
+    TileWalk walk;
+    walk.ntiles = ntiles;
+    walk.K = K;
     if (dyn) {
         if (threadIdx.x == 0) *grab = atomicAdd(P.rc_tile_next, K);
         __syncthreads();
-        t = *grab;
-        tend = min(t + K, ntiles);
+        walk.enter(*grab);
         __syncthreads();                        // every thread has read it before the next grab
     } else {
-        t = (int)((long long)ntiles * blockIdx.x / gridDim.x);
-        tend = (int)((long long)ntiles * (blockIdx.x + 1) / gridDim.x);
+        walk.t = (int)((long long)ntiles * blockIdx.x / gridDim.x);
+        walk.end = (int)((long long)ntiles * (blockIdx.x + 1) / gridDim.x);
     }
-    if (t >= tend) return;
+    if (walk.t >= walk.end) return;
     const int warp = threadIdx.x >> 5, l32 = threadIdx.x & 31;
     const int lane = l32 % T;
     // the columns of a warp: all even or all odd, this team's at 4 times tms;
@@ -892,15 +894,16 @@ __global__ void __launch_bounds__(THR, MINB) k_cols_rcp(Plan P) {
         cp_async_commit();
     };
 
-    stage_slave(t);
-    stage_master(t);
+    stage_slave(walk.t);
+    stage_master(walk.t);
 
     int cur_w = -1;
     for (;;) {
         int w, b;
+        const int t = walk.t;
         tile(t, w, b);
         // the last tile of a chunk: the next chunk, read after the barrier below
-        if (dyn && t + 1 == tend && threadIdx.x == 0) *grab = atomicAdd(P.rc_tile_next, K);
+        if (dyn && walk.last() && threadIdx.x == 0) *grab = atomicAdd(P.rc_tile_next, K);
         const int kx0 = b * CP;
         const bool neww = (w != cur_w);
         // (the previous tile's last barrier ordered every read of boxx and dsum before these writes)
@@ -917,9 +920,7 @@ __global__ void __launch_bounds__(THR, MINB) k_cols_rcp(Plan P) {
         }
         cp_async_wait<1>();                      // this tile's slave rows in (this thread's copies)
         __syncthreads();                         // ... and everyone's; boxx, dsum, tw, boxy, grab written
-        int tn = -1;                             // the next tile, none: -1
-        if (t + 1 < tend) tn = t + 1;
-        else if (dyn && *grab < ntiles) tn = *grab;
+        const int tn = walk.next(dyn && walk.last() ? *grab : ntiles);      // the next tile, none: -1
         if (neww && warp == 0) {                 // one warp: GB300 issues two FP64 operations per SM and cycle
             const double inv = pow2_inv(N * M);
             const double s1 = (dsum[0] + dsum[1]) * inv, s2 = (dsum[2] + dsum[3]) * inv;
@@ -1061,8 +1062,7 @@ __global__ void __launch_bounds__(THR, MINB) k_cols_rcp(Plan P) {
         if (tn < 0) break;
         if (b == 0) stage_slave(tn);
         stage_master(tn);
-        if (tn != t + 1) tend = min(tn + K, ntiles);
-        t = tn;
+        walk.go(tn);
     }
 }
 
