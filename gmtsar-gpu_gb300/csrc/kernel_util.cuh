@@ -60,33 +60,24 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int NPEND>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(NPEND) : "memory"); }
 
-// Programmatic dependent launch: a kernel launched by launch_chain may start
-// while the one before it in its stream still runs; grid_dep_wait returns once
-// that one has completed with its writes visible (at once in a kernel that was
-// launched the ordinary way), and grid_dep_launch lets the next one start as
-// soon as every CTA of this one has called it or left.
+// Programmatic dependent launch: a kernel launched by launch_chain starts when
+// the last CTA of the one before it in its stream leaves, instead of when that
+// one has completed; grid_dep_wait returns once it has, with its writes visible
+// (at once in a kernel that was launched the ordinary way).
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
-// The kernels of a batch are launched as programmatic dependents (P.chain).
-// 1, a batch alone on its stream: every kernel lets the next one start at its
-// own start, so that each is resident with its tables staged when the one
-// before it ends: one strip of 20 windows 61.5 -> 55.7 us.  2, several batches
-// in flight: waiting CTAs would take the slots of the other batches' kernels,
-// so the next kernel starts when the last CTA of this one leaves; what is saved
-// is the launch: 1000 windows 401 -> 395 us, through host buffers 578 -> 566.
-// (Starting it during the last tile measured the same.)
-// A batch alone also asks for the largest shared-memory split from its first
-// kernel (dependent = false) on: an SM changes its split only when it is idle,
-// so a kernel of another split could not start beside the one before it (the
-// strip: 51.8 -> 48.4 us).  With several batches the same split would mix their
-// row and column kernels on an SM, which costs (40,000 windows of 256 x 256:
-// 54.8 -> 61.8 ms), so they keep the splits of their own sizes.  3, a lone batch's
-// row bands, which wait for their copies: plain launches with that split.
+// The kernels of a batch are launched as programmatic dependents (P.chain): what
+// is saved is the launch, 1000 windows 401 -> 395 us, through host buffers 578 ->
+// 566.  A kernel neither lets the next one start before its last CTA leaves nor
+// asks for a larger shared-memory split than its own: waiting CTAs and a common
+// split take room from whatever runs beside, another batch or another context's
+// call.  With both, a lone batch of 80 windows of 128 x 128 took 95 us where it
+// takes 87, from four contexts at once 68 where it takes 60 (66 before there were
+// dependents), 391 windows of 128 x 64 215 against 207 and a strip of 20 of 128 x
+// 128 47.0 against 43.9.
 template <class Kernel>
-inline void launch_chain(const Plan &P, Kernel kern, dim3 grid, int threads, size_t smem, cudaStream_t s, int cluster = 1,
-                         bool dependent = true) {
-    if (P.chain == 0 && cluster == 1) {
+inline void launch_chain(const Plan &P, Kernel kern, dim3 grid, int threads, size_t smem, cudaStream_t s, int cluster = 1) {
+    if (!P.chain && cluster == 1) {
         kern<<<grid, threads, smem, s>>>(P);
         return;
     }
@@ -95,13 +86,9 @@ inline void launch_chain(const Plan &P, Kernel kern, dim3 grid, int threads, siz
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute at[3];
+    cudaLaunchAttribute at[2];
     cfg.attrs = at;
-    if (P.chain & 1) {
-        at[cfg.numAttrs].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
-        at[cfg.numAttrs++].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
-    }
-    if ((P.chain == 1 || P.chain == 2) && dependent) {
+    if (P.chain) {
         at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
     }

@@ -123,7 +123,6 @@ __device__ __forceinline__ void warp_sort(unsigned long long &k, int &p) {
 template <int NT, int PER>
 __global__ void __launch_bounds__(NT, 1) k_rc_plan(Plan P) {
     const int tid = threadIdx.x;
-    if (P.chain == 1) grid_dep_launch();
     // Two CTAs (no row bands): CTA i plans image i's entries alone, its runs
     // never meeting the other image's, and numbers its chunks from
     // i * nwin * nchunks (the most chunks the master entries can need), so
@@ -390,7 +389,6 @@ __global__ void __launch_bounds__(128, (N >= 1024) ? 2 : (N >= 512 ? 3 : 4)) k_s
     // KEEPS: each thread's spectrum elements, [PER][32] per warp
     float2 *spec = reinterpret_cast<float2 *>(after) + (size_t)warp * PER * 32 + l32;
 
-    if (P.chain == 1) grid_dep_launch();
     for (int i = threadIdx.x; i < TWL; i += blockDim.x) tw[i] = P.tw_row[i];
     if constexpr (HSHIFT)
         for (int i = threadIdx.x; i < TWL; i += blockDim.x) tw[TWL + i] = P.phase[i];
@@ -833,7 +831,6 @@ __global__ void __launch_bounds__(THR, MINB) k_cols_rcp(Plan P) {
     // call in single tiles).  Shorter chunks towards the end of a large batch
     // cost more in patch means than the shorter tail gives (1000 windows of
     // 128 x 128: 426 against 420 us).
-    if (P.chain == 1) grid_dep_launch();
     for (int i = threadIdx.x; i < TWL; i += THR) cp_async8(tw + i, P.tw_col + i);
     for (int i = threadIdx.x; i < M; i += THR) cp_async8(boxy + i, P.box_y + i);
     cp_async_commit();               // a group of its own, complete when the first tile's slave rows are
@@ -1168,9 +1165,9 @@ void launch_rc_plan(const Plan &P, cudaStream_t s) {
     // one CTA per image unless the host entry wants the chunks listed by row band
     const int ctas = P.rc_nbands > 0 ? 1 : 2, nent = ctas == 1 ? 2 * P.nwin : P.nwin;
     const size_t sm = rc_plan_smem_bytes(nent);
-    if (nent <= 128) launch_chain(P, k_rc_plan<128, 1>, dim3(ctas), 128, sm, s, 1, false);
-    else if (nent <= 512) launch_chain(P, k_rc_plan<512, 1>, dim3(ctas), 512, sm, s, 1, false);
-    else launch_chain(P, k_rc_plan<512, RC_ENTRIES / 512>, dim3(ctas), 512, sm, s, 1, false);
+    if (nent <= 128) k_rc_plan<128, 1><<<ctas, 128, sm, s>>>(P);
+    else if (nent <= 512) k_rc_plan<512, 1><<<ctas, 512, sm, s>>>(P);
+    else k_rc_plan<512, RC_ENTRIES / 512><<<ctas, 512, sm, s>>>(P);
 }
 
 template <int N, bool SPEC = true>

@@ -581,7 +581,7 @@ xcg_status ctx_launch(xcg_ctx *c, Plan P, const int *starts, int nb, cudaStream_
     P.chain = 0;
     if (rc && P.corr_mode == 2 && c->profiling == 0 && P.cols_cfg != 1) {
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusActive;
-        if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) P.chain = nb == 1 ? 1 : 2;
+        if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) P.chain = 1;
     }
     if (P.corr_mode < 2) {
         P.time_giveup = c->inject_tc_timeout;
@@ -857,7 +857,7 @@ xcg_status xcg_correlate(xcg_ctx *c, const void *master, int32_t m_nx, int32_t m
             int lo[2], hi[2];
             for (int k = 0; k < 2; k++) rows_of(Q.win0, Q.win0 + Q.nwin, k, lo[k], hi[k]);
             xcg::Plan Qb = Q;
-            Qb.chain = (Q.chain == 1) ? 3 : 0;      // a band's rows wait for its copy, not only for the launch before
+            Qb.chain = 0;               // a band's rows wait for its copy, not only for the launch before
             const int nb = std::max(1, std::min(8, Q.nwin / 128));
             Qb.rc_nbands = nb;
             for (int b = 0; b < nb; b++)

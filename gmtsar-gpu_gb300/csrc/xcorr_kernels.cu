@@ -544,7 +544,6 @@ __global__ void __launch_bounds__(NT, MINB) k_peak(Plan P) {
         }
         cp_async_commit();
     };
-    if (P.chain == 1) grid_dep_launch();
     for (int i = threadIdx.x; i < TWL; i += NT) cp_async8(tw + i, P.tw_row + i);
     cp_async_commit();
     grid_dep_wait();                                      // the column stage's half spectra
@@ -895,7 +894,6 @@ __global__ void __launch_bounds__(256, 4) k_subpix(Plan P) {
     __shared__ int holder[NT];
 
     const int w = blockIdx.x, tid = threadIdx.x;
-    if (P.chain == 1) grid_dep_launch();
     for (int t = tid; t < NX2 * N2 / 2; t += NT) cp_async16(kys + 2 * t, P.ky + 2 * t);
     cp_async_commit();
     float4 kx[XT][4];                                 // two entries of the row operator's row X per vector

@@ -84,7 +84,7 @@ struct Plan {
     // row segment that one or more windows of the batch read, in chunks of
     // 1024 samples; a window's patch rows are consecutive rows of its chunks
     int rc;                 // 1: this path; 0: one row stage per window (zrow, amp1, ...)
-    int chain;              // how the batch's kernels follow each other (launch_chain): 0, 3 plain launches, 1, 2 dependents
+    int chain;              // 1: the batch's kernels are launched as dependents of each other (launch_chain); 0: plainly
     int rpc;                // rows per chunk: 1024 / npx
     int4 *rc_desc;          // [chunks] (pair, 0 master / 1 slave, first column, first row)
     int2 *rc_wch;           // [nwin] first master (x) and slave (y) chunk of each window
