@@ -575,6 +575,7 @@ xcg_status ctx_launch(xcg_ctx *c, Plan P, const int *starts, int nb, cudaStream_
     const int lanes = mode ? 2 * c->nslots : c->nslots;
     const bool fork = nb > 1 && lanes > 1 && c->profiling != 1;
     const bool tl = c->profiling == 2;
+    P.batches = nb;
     // the kernels of a batch chained as programmatic dependents (not while
     // profiling, whose events lie between them, nor into a captured graph,
     // which keeps plain kernel edges)

@@ -1082,12 +1082,25 @@ static size_t cols_smem(int) {
     using G = ColsGeom<M, THR>;
     return G::TWL * sizeof(float2) + (size_t)2 * G::CP * G::CS * sizeof(float2) + 2 * sizeof(double);
 }
-// A cluster of four CTAs per window while all of them fit the GPU at once (four
-// per SM) and each rank's teams have a row pair: with their launches, 20
-// windows of 128 x 128 22.2 -> 14.9 us, 140 of them 24.6 -> 22.6, 20 of 256 x
-// 256 57 -> 26.5.  More windows hide each other's latency (200: the same), and
-// ranks without rows only wait (100 windows of 64 x 64: 14.3 -> 18.4 us).
-constexpr int PEAK_CL = 4, PEAK_CL_WINDOWS = 152;
+// A cluster of four CTAs per window for batches that leave the GPU room: each
+// window's latency falls (the stage with its launch: 20 windows of 128 x 128 22.2
+// -> 14.9 us, 140 of them 24.6 -> 22.6, 20 of 256 x 256 57 -> 26.5), but a cluster
+// starts only where four places are free at once, and ranks without a row pair
+// only wait (100 windows of 64 x 64: 14.3 -> 18.4 us).  The most windows of a
+// batch, alone and with another batch of its call in flight, by the transform's
+// length, from whole calls with and without clusters (us):
+//   up to 256 points  152 alone: 152 of 128 x 128 151 against 154.  100 beside
+//                     another: 200 in two batches 172 against 177; 300 in two 217
+//                     against 216, and from four contexts at once 204 against 187
+//                     (195 before there were clusters)
+//   512               152 both: 152 of 256 x 256 327 against 367, 300 in two batches
+//                     495 against 505
+//   1024 (one CTA     72 alone: 72 of 512 x 128 305 against 312, 76 317 against 315,
+//   per SM)           120 388 against 366.  38 beside another: 72 in two batches 292
+//                     against 303, 76 308 against 308, 120 360 against 344
+constexpr int PEAK_CL = 4;
+template <int N>
+constexpr int peak_cl_windows(bool alone) { return N <= 256 ? (alone ? 152 : 100) : N <= 512 ? 152 : (alone ? 72 : 38); }
 // resident k_peak CTAs per SM for configuration cfg
 template <int N>
 constexpr int peak_minb(int cfg) { return (N <= 256) ? (cfg == 1 ? 3 : 4) : (N <= 512 ? (cfg == 1 ? 2 : 3) : 1); }
@@ -1196,7 +1209,7 @@ static void launch_cols_t(const Plan &P, cudaStream_t s) {
 }
 template <int N>
 static void launch_peak_t(const Plan &P, cudaStream_t s) {
-    if (P.nwin <= PEAK_CL_WINDOWS && P.nyc / 2 >= PEAK_CL * (256 / fft_lanes(N)) && P.peak_cfg == 0) {
+    if (P.nwin <= peak_cl_windows<N>(P.batches <= 1) && P.nyc / 2 >= PEAK_CL * (256 / fft_lanes(N)) && P.peak_cfg == 0) {
         launch_chain(P, k_peak<N, peak_minb<N>(0), 256, PEAK_CL>, dim3(P.nwin * PEAK_CL), 256, peak_smem<N>(), s, PEAK_CL);
         return;
     }

@@ -54,6 +54,7 @@ struct Plan {
     // windows of this batch
     const xcg_loc *locs;   // already offset to the batch's first window
     int nwin;              // windows in this batch
+    int batches;           // batches of the call, which may be in flight at once
     int win0;              // single pair: index of the batch's first window
 
     // tables (device, built on the host in double)

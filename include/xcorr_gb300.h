@@ -243,11 +243,15 @@ xcg_status xcg_set_row_sharing(xcg_ctx *ctx, int32_t enable);
  * counter, the next tile's rows staged during the current one, in the
  * faster form for the size (up to 512-point columns the slave's column
  * spectrum kept in registers at one CTA per SM fewer, 512-point columns by
- * 16 lanes each); 1 one CTA per tile; 2 persistent in the other form.  Without sharing: 0 128-thread CTAs, two cp.async staging groups;
- * 1 256-thread CTAs; 2 one staging group.  peak_cfg: 0 four CTAs per SM of
- * 256 threads per window (three for 512-point transforms), 1 one fewer,
- * 2 512 threads per window (transforms up to 512 points; the others take
- * 0).  Every shape gives the same bits. */
+ * 16 lanes each); 1 one CTA per tile; 2 persistent in the other form.  Without
+ * sharing: 0 128-thread CTAs, two cp.async staging groups; 1 256-thread CTAs;
+ * 2 one staging group.  peak_cfg: 0 CTAs of 256 threads, four per SM (three for
+ * 512-point transforms, one for 1024), one per window, or a cluster of four per
+ * window in batches of up to 152 windows (72 for 1024 points; beside another
+ * batch of the call 100 up to 256 points, 38 for 1024) where the surface has a
+ * row pair for every team of the cluster; 1 always one CTA per window, one fewer
+ * per SM where 0 has several; 2 one CTA of 512 threads per window (transforms up
+ * to 512 points; for 1024 one of 256).  Every shape gives the same bits. */
 xcg_status xcg_set_launch_shapes(xcg_ctx *ctx, int32_t cols_cfg, int32_t peak_cfg);
 
 /* Split each later call's windows into this many batches (whole strips; at
