@@ -33,7 +33,6 @@ namespace {
 namespace cg = cooperative_groups;
 
 constexpr int FIT_THREADS = 256;
-constexpr int FIT_CTAS = 16;   // CTAs per axis: one cluster
 constexpr int NS = 10;         // per axis: w, wu, wv, wuu, wuv, wvv, wo, wuo, wvo, woo
 // points a CTA keeps in shared memory between passes (u, v, o: 20 bytes
 // each); a call's further points are formed again from the records each pass
@@ -89,7 +88,7 @@ __device__ __forceinline__ int split_slot(int lane) {
     return (n >= 1 && (lane & 1) == 0) ? lo : -1;
 }
 
-// One cluster of 16 CTAs per axis (the axes share nothing but the points
+// One cluster of CTAS CTAs per axis (the axes share nothing but the points
 // used).  GB300 issues two FP64 operations per SM and cycle, and a pass is
 // about 20 of them per point and axis, so the FP64 pipe bounds the fit: one
 // CTA for both axes took 3466 us for 40,000 points and four passes; 2 x 16
@@ -97,6 +96,7 @@ __device__ __forceinline__ int split_slot(int lane) {
 // by reciprocals instead of divisions and a split reduction take 92 us.  A
 // cluster's barriers order the passes, so there is no workspace in device
 // memory: calls on several streams stay independent.
+template <int CTAS>
 __global__ void __launch_bounds__(FIT_THREADS, 1) k_fit(const xcg_result *__restrict__ res, const xcg_loc *__restrict__ locs,
                                                      int n, int ri, int x_offset, int y_offset, double astretcha,
                                                      float snr_min, int npar_r, int npar_a, int robust_iters, int keep,
@@ -111,9 +111,9 @@ __global__ void __launch_bounds__(FIT_THREADS, 1) k_fit(const xcg_result *__rest
     __shared__ double total[NS];
     __shared__ AxisModel mod;
     cg::cluster_group cl = cg::this_cluster();
-    const int rank = (int)cl.block_rank(), axis = (int)blockIdx.x / FIT_CTAS;
+    const int rank = (int)cl.block_rank(), axis = (int)blockIdx.x / CTAS;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int stride = FIT_CTAS * FIT_THREADS, first = rank * FIT_THREADS + (int)threadIdx.x;
+    const int stride = CTAS * FIT_THREADS, first = rank * FIT_THREADS + (int)threadIdx.x;
 
     // pass 0: extent of the used locations; a point left out is kept as NaN
     int e0 = INT32_MAX, e1 = INT32_MIN, e2 = INT32_MAX, e3 = INT32_MIN, cnt = 0;
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(FIT_THREADS, 1) k_fit(const xcg_result *__rest
     }
     cl.sync();
     e0 = INT32_MAX; e1 = INT32_MIN; e2 = INT32_MAX; e3 = INT32_MIN; cnt = 0;
-    for (int r = 0; r < FIT_CTAS; r++) {
+    for (int r = 0; r < CTAS; r++) {
         const int *q = cl.map_shared_rank(ext, r);
         e0 = min(e0, q[0]); e1 = max(e1, q[1]); e2 = min(e2, q[2]); e3 = max(e3, q[3]); cnt += q[4];
     }
@@ -224,11 +224,11 @@ __global__ void __launch_bounds__(FIT_THREADS, 1) k_fit(const xcg_result *__rest
         }
         cl.sync();             // the parity keeps a slow CTA's reads apart from the next pass's sums
         if (threadIdx.x < NS) {
-            double s[FIT_CTAS];
+            double s[CTAS];
 #pragma unroll
-            for (int r = 0; r < FIT_CTAS; r++) s[r] = cl.map_shared_rank(part[pass & 1], r)[threadIdx.x];
+            for (int r = 0; r < CTAS; r++) s[r] = cl.map_shared_rank(part[pass & 1], r)[threadIdx.x];
 #pragma unroll
-            for (int h = FIT_CTAS / 2; h > 0; h /= 2)
+            for (int h = CTAS / 2; h > 0; h /= 2)
 #pragma unroll
                 for (int r = 0; r < h; r++) s[r] += s[r + h];
             total[threadIdx.x] = s[0];
@@ -268,42 +268,95 @@ __global__ void __launch_bounds__(FIT_THREADS, 1) k_fit(const xcg_result *__rest
 
 constexpr size_t fit_smem(int keep) { return (size_t)keep * (2 * sizeof(double) + sizeof(float)); }
 
-}  // namespace
+struct FitCall {
+    const xcg_result *res;
+    const xcg_loc *locs;
+    int n, ri, x_offset, y_offset;
+    double astretcha;
+    float snr_min;
+    int npar_range, npar_azimuth, robust_iters;
+    xcg_fit *out;
+    cudaStream_t stream;
+};
 
-extern "C" xcg_status xcg_fit_offsets(const xcg_result *d_results, const xcg_loc *d_locs, int32_t nlocs, int32_t ri,
-                                      int32_t x_offset, int32_t y_offset, double astretcha, float snr_min,
-                                      int32_t npar_range, int32_t npar_azimuth, int32_t robust_iters, xcg_fit *d_out,
-                                      void *stream) {
-    if (!d_results || !d_locs || !d_out || nlocs < 0 || ri < 1 || npar_range < 1 || npar_range > 3 ||
-        npar_azimuth < 1 || npar_azimuth > 3 || robust_iters < 0 || robust_iters > 100) {
+// Launches the fit on clusters of CTAS CTAs; with `ask`, only where the device
+// has room for such a cluster (ran: whether it was launched).
+template <int CTAS>
+cudaError_t launch_fit(const FitCall &f, bool ask, bool &ran) {
+    ran = false;
+    // the kernel's attributes, per device (idempotent: every call may set them)
+    cudaError_t e = CTAS > 8 ? cudaFuncSetAttribute(k_fit<CTAS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) : cudaSuccess;
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_fit<CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fit_smem(FIT_KEEP));
+    if (e != cudaSuccess) return e;
+    const long long per = (long long)CTAS * FIT_THREADS;           // points a cluster takes at a time
+    const int keep = (int)std::min<long long>(FIT_KEEP, (f.n + per - 1) / per * FIT_THREADS);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * CTAS);
+    cfg.blockDim = dim3(FIT_THREADS);
+    cfg.dynamicSmemBytes = fit_smem(keep);
+    cfg.stream = f.stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = CTAS;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (ask) {
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, k_fit<CTAS>, &cfg) != cudaSuccess) {
+            cudaGetLastError();        // not an error of the call: the next form is tried
+            clusters = 0;
+        }
+        if (clusters < 1) return cudaSuccess;
+    }
+    ran = true;
+    return cudaLaunchKernelEx(&cfg, k_fit<CTAS>, f.res, f.locs, f.n, f.ri, f.x_offset, f.y_offset, f.astretcha, f.snr_min,
+                              f.npar_range, f.npar_azimuth, f.robust_iters, keep, f.out);
+}
+
+// ctas: CTAs per axis, 16, 8 or 1; 0: the most of them that fit.  A cluster lies
+// in one GPC, and a part of a GPU (an instance, a partition) may have none with
+// 16 SMs free for it.  The same sums in another order.
+xcg_status fit_offsets(const FitCall &f, int ctas) {
+    if (!f.res || !f.locs || !f.out || f.n < 0 || f.ri < 1 || f.npar_range < 1 || f.npar_range > 3 || f.npar_azimuth < 1 ||
+        f.npar_azimuth > 3 || f.robust_iters < 0 || f.robust_iters > 100) {
         xcg::set_last_error("xcg_fit_offsets: invalid argument");
         return XCG_ERR_ARG;
     }
-    // the kernel's attributes, per device (idempotent: every call may set them)
-    cudaError_t e = cudaFuncSetAttribute(k_fit, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_fit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fit_smem(FIT_KEEP));
-    if (e == cudaSuccess) {
-        const long long per = (long long)FIT_CTAS * FIT_THREADS;       // points a cluster takes at a time
-        const int keep = (int)std::min<long long>(FIT_KEEP, (nlocs + per - 1) / per * FIT_THREADS);
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(2 * FIT_CTAS);
-        cfg.blockDim = dim3(FIT_THREADS);
-        cfg.dynamicSmemBytes = fit_smem(keep);
-        cfg.stream = (cudaStream_t)stream;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = FIT_CTAS;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        e = cudaLaunchKernelEx(&cfg, k_fit, d_results, d_locs, (int)nlocs, (int)ri, (int)x_offset, (int)y_offset, astretcha,
-                               snr_min, (int)npar_range, (int)npar_azimuth, (int)robust_iters, keep, d_out);
-    }
+    const bool any = ctas == 0;
+    bool ran = false;
+    cudaError_t e = cudaSuccess;
+    if (any || ctas == 16) e = launch_fit<16>(f, any, ran);
+    if (e == cudaSuccess && !ran && (any || ctas == 8)) e = launch_fit<8>(f, any, ran);
+    if (e == cudaSuccess && !ran && (any || ctas == 1)) e = launch_fit<1>(f, false, ran);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) {
         xcg::set_last_error(cudaGetErrorString(e));
         return XCG_ERR_CUDA;
     }
     return XCG_OK;
+}
+
+}  // namespace
+
+extern "C" xcg_status xcg_fit_offsets(const xcg_result *d_results, const xcg_loc *d_locs, int32_t nlocs, int32_t ri,
+                                      int32_t x_offset, int32_t y_offset, double astretcha, float snr_min,
+                                      int32_t npar_range, int32_t npar_azimuth, int32_t robust_iters, xcg_fit *d_out,
+                                      void *stream) {
+    return fit_offsets({d_results, d_locs, nlocs, ri, x_offset, y_offset, astretcha, snr_min, npar_range, npar_azimuth,
+                        robust_iters, d_out, (cudaStream_t)stream}, 0);
+}
+
+extern "C" xcg_status xcg_debug_fit_offsets(int32_t ctas, const xcg_result *d_results, const xcg_loc *d_locs, int32_t nlocs,
+                                            int32_t ri, int32_t x_offset, int32_t y_offset, double astretcha, float snr_min,
+                                            int32_t npar_range, int32_t npar_azimuth, int32_t robust_iters,
+                                            xcg_fit *d_out, void *stream) {
+    if (ctas != 1 && ctas != 8 && ctas != 16) {
+        xcg::set_last_error("xcg_debug_fit_offsets: 1, 8 or 16 CTAs per axis");
+        return XCG_ERR_ARG;
+    }
+    return fit_offsets({d_results, d_locs, nlocs, ri, x_offset, y_offset, astretcha, snr_min, npar_range, npar_azimuth,
+                        robust_iters, d_out, (cudaStream_t)stream}, ctas);
 }

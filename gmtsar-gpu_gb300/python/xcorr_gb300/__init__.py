@@ -27,7 +27,7 @@ EXPORTS = ("xcg_status_string", "xcg_last_error", "xcg_default_params", "xcg_cre
            "xcg_stack_autotune", "xcg_stack_get_stats", "xcg_set_features", "xcg_refiner_create",
            "xcg_refiner_destroy", "xcg_refiner_set_params", "xcg_refiner_get_params", "xcg_refiner_forward",
            "xcg_refiner_gradient", "xcg_refiner_train_step", "xcg_correlate_device_refined",
-           "xcg_fit_offsets", "xcg_tc_gemm_check", "xcg_set_dft_form", "xcg_debug_inject_stage_timeout",
+           "xcg_fit_offsets", "xcg_debug_fit_offsets", "xcg_tc_gemm_check", "xcg_set_dft_form", "xcg_debug_inject_stage_timeout",
            "xcg_fp32_fma_rate", "xcg_set_row_sharing", "xcg_set_launch_shapes", "xcg_set_batches")
 REFINER_NPARAM = 37507
 FLAG_REFINED = 4
@@ -164,6 +164,7 @@ def load(path: str | None = None):
     L.xcg_fit_offsets.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
                                   ctypes.c_int32, ctypes.c_double, ctypes.c_float, ctypes.c_int32, ctypes.c_int32,
                                   ctypes.c_int32, ctypes.c_void_p, ctypes.c_void_p]
+    L.xcg_debug_fit_offsets.argtypes = [ctypes.c_int32] + L.xcg_fit_offsets.argtypes
     L.xcg_tc_gemm_check.argtypes = [ctypes.c_int32] * 4 + [ctypes.c_void_p] * 4
     L.xcg_set_dft_form.argtypes = [ctypes.c_void_p, ctypes.c_int32]
     L.xcg_debug_inject_stage_timeout.argtypes = [ctypes.c_void_p]
@@ -402,12 +403,14 @@ def correlate_device_noalloc(p: Params, d_master: int, m_nx: int, m_ny: int, d_s
 
 
 def fit_offsets(d_results: int, d_locs: int, nlocs: int, d_out: int, ri=2, x_offset=0, y_offset=0, astretcha=0.0,
-                snr_min=20.0, npar_range=3, npar_azimuth=3, robust_iters=0, stream: int = 0):
+                snr_min=20.0, npar_range=3, npar_azimuth=3, robust_iters=0, stream: int = 0, ctas: int = 0):
     """xcg_fit_offsets: the PRM offset model fitted on the device from a
-    device result array; d_out is a device buffer of sizeof(Fit) bytes."""
+    device result array; d_out is a device buffer of sizeof(Fit) bytes.  ctas:
+    16, 8 or 1 CTAs per axis (xcg_debug_fit_offsets), 0 the most that fit."""
     L = load()
-    _check(L.xcg_fit_offsets(d_results, d_locs, int(nlocs), int(ri), int(x_offset), int(y_offset), float(astretcha),
-                             float(snr_min), int(npar_range), int(npar_azimuth), int(robust_iters), d_out, stream))
+    args = (d_results, d_locs, int(nlocs), int(ri), int(x_offset), int(y_offset), float(astretcha), float(snr_min),
+            int(npar_range), int(npar_azimuth), int(robust_iters), d_out, stream)
+    _check(L.xcg_debug_fit_offsets(int(ctas), *args) if ctas else L.xcg_fit_offsets(*args))
 
 
 def tc_gemm_check(m_tiles: int, n_tile: int, k: int, n_total: int, d_a: int, d_b: int, d_c: int, stream: int = 0):

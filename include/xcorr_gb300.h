@@ -331,6 +331,13 @@ xcg_status xcg_fit_offsets(const xcg_result *d_results, const xcg_loc *d_locs, i
                            int32_t npar_range, int32_t npar_azimuth, int32_t robust_iters, xcg_fit *d_out,
                            void *stream);
 
+/* Diagnostic: xcg_fit_offsets on 16, 8 or 1 CTAs per axis, of which it takes the
+ * most that the device has room for. */
+xcg_status xcg_debug_fit_offsets(int32_t ctas, const xcg_result *d_results, const xcg_loc *d_locs, int32_t nlocs,
+                                 int32_t ri, int32_t x_offset, int32_t y_offset, double astretcha, float snr_min,
+                                 int32_t npar_range, int32_t npar_azimuth, int32_t robust_iters, xcg_fit *d_out,
+                                 void *stream);
+
 /* DFT form of the frequency-domain path: 0 (default) FP32 SIMT team FFTs; 1
  * the precision form, in which the forward row and column DFTs of the 2-D
  * correlation and the inverse column DFT of the product run as split-FP16
