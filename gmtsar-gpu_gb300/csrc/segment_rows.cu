@@ -54,6 +54,9 @@ constexpr int RC_ENTRIES = 2 * RC_MAX_WINDOWS;   // sort capacity, a power of tw
 constexpr int KEY_Y_BITS = 24;
 constexpr int KEY_Y_BIAS = 1 << 23;
 constexpr int KEY_X_BIAS = 1 << 19;
+bool rc_fits(const PairDev &p) {
+    return std::max(p.m_nx, p.s_nx) < KEY_X_BIAS && std::max(p.m_ny, p.s_ny) < KEY_Y_BIAS;
+}
 
 // In-place exclusive scan of a[0, ns) by the whole CTA (ns a multiple of NT,
 // at most PER_THREAD of them); returns the total.
@@ -153,8 +156,12 @@ __global__ void __launch_bounds__(NT, 1) k_rc_plan(Plan P) {
             const xcg_loc loc = P.locs[w];
             int local, pidx;
             const PairDev pd = pair_of(P, w, local, pidx);
-            const int x0 = img ? loc.x + pd.x_offset - npx / 2 : loc.x - npx / 2;
-            const int y0 = img ? loc.y + pd.y_offset + slave_row_shift(pd, loc.y) - npy / 2 : loc.y - npy / 2;
+            int x0 = img ? loc.x + pd.x_offset - npx / 2 : loc.x - npx / 2;
+            int y0 = img ? loc.y + pd.y_offset + slave_row_shift(pd, loc.y) - npy / 2 : loc.y - npy / 2;
+            // a patch wholly outside its image is the same wherever it lies: at
+            // the image's edge its place fits the key (rc_fits)
+            x0 = min(max(x0, -npx), img ? pd.s_nx : pd.m_nx);
+            y0 = min(max(y0, -npy), img ? pd.s_ny : pd.m_ny);
             const int ym = ((y0 % rpc) + rpc) % rpc;
             k = ((unsigned long long)pidx << 49) | ((unsigned long long)img << 48) |
                 ((unsigned long long)(x0 + KEY_X_BIAS) << 28) | ((unsigned long long)ym << KEY_Y_BITS) |

@@ -493,6 +493,7 @@ Plan rows_subrange(Plan P, int off, int n) {
 // million pixels that barely overlap: 536 -> 550).
 static bool shares_rows(const Plan &P, int nlocs) {
     if (!P.rc || P.tc_form) return false;             // the precision form reads the per-window arrays
+    if (!P.pairs && !rc_fits(P.single)) return false; // (a stack's pairs: its plan)
     return P.corr_mode == 2 || (size_t)nlocs * P.npx * P.npy >= ((size_t)1 << 24);
 }
 
