@@ -487,14 +487,20 @@ Plan rows_subrange(Plan P, int off, int n) {
 }
 
 // Whether a job of nlocs windows runs on shared row segments.  In the -time and
-// -time4 modes from 2^24 pixels of patches on: the row stage per window takes 5 to 7
-// us per million, and sharing has a planner to pay (17 us) however little the
-// windows overlap (1000 windows of 128 x 128: 3037 -> 2828 us; 400 of 64 x 64, 6.5
-// million pixels that barely overlap: 536 -> 550).
+// -time4 modes from 2^24 pixels of patches on, in patches of 2^15 or more: the row
+// stage per window takes 5 to 7 us per million, and sharing has planners to pay
+// (17 to 55 us) however little the windows overlap.  1000 windows of 128 x 128
+// 2978 us per window, 2753 shared where rows belong to 3.6 patches, 2992 and 2972
+// where none does; 400 of 64 x 64, 6.5 million pixels that barely overlap, 536 and
+// 550; 576 of 128 x 64 without overlap 919 and 927, 1000 of them at 3.6 1542 and
+// 1451.  Smaller patches have eight rows to a chunk, and only patches whose first
+// rows agree modulo eight share one: 1040 of 64 x 64 666 and 766, 1200 of them at
+// 4.3 741 and 795, 2000 without overlap 1247 and 1320 (2048 at 10.7 1232 and 1185).
 static bool shares_rows(const Plan &P, int nlocs) {
     if (!P.rc || P.tc_form) return false;             // the precision form reads the per-window arrays
     if (!P.pairs && !rc_fits(P.single)) return false; // (a stack's pairs: its plan)
-    return P.corr_mode == 2 || (size_t)nlocs * P.npx * P.npy >= ((size_t)1 << 24);
+    const size_t patch = (size_t)P.npx * P.npy;
+    return P.corr_mode == 2 || (patch >= ((size_t)1 << 15) && nlocs * patch >= ((size_t)1 << 24));
 }
 
 int ctx_batch_windows(const xcg_ctx *c, int nlocs, int strip_len) {
