@@ -48,10 +48,6 @@ __device__ __forceinline__ void cp_async8(void *smem, const void *gmem) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(gmem) : "memory");
 }
-__device__ __forceinline__ void cp_async4(void *smem, const void *gmem) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(gmem) : "memory");
-}
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {   // 16-byte aligned both
     const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmem) : "memory");

@@ -18,8 +18,7 @@ constexpr int RP_W1 = 0, RP_B1 = 288, RP_W2 = 320, RP_B2 = 9536, RP_W3 = 9568, R
 // with channels 12 apart.  Every section starts on 16 bytes.
 constexpr int A1_CS = 60, A2_CS = 44, A1_LEN = 32 * A1_CS, A2_LEN = 32 * A2_CS;
 constexpr int ACT_A1 = 0, ACT_A2 = ACT_A1 + A1_LEN, ACT_A3 = ACT_A2 + A2_LEN, ACT_G1 = ACT_A3 + 288, ACT_D1 = ACT_G1 + 64,
-              ACT_D2 = ACT_D1 + 32 * 56, ACT_D3 = ACT_D2 + 32 * 40, ACT_DZ = ACT_D3 + 288, ACT_OUT = ACT_DZ + 64,
-              REF_ACT = ACT_OUT + 4;
+              ACT_D2 = ACT_D1 + 32 * 56, ACT_D3 = ACT_D2 + 32 * 40, REF_ACT = ACT_D3 + 288;
 constexpr int GRD_Y1 = 0, GRD_Y2 = A1_LEN, GRD_Y3 = GRD_Y2 + 32 * 40, GRD_Z = GRD_Y3 + 32 * 12, GRD_OUT = GRD_Z + 64,
               REF_GRAD = GRD_OUT + 4;
 constexpr int REF_SMS = 152;         // CTAs of a full training launch: one per SM

@@ -129,10 +129,6 @@ __device__ __forceinline__ int demeaned_int(float amp, float mean) {
 
 // ------------------------------------------------------------------ k_tprep
 
-// Slab width (columns of the window per pass of k_tcorr_tc) and tile width of
-// a window geometry; see tc_geom below for the shared memory they come from.
-struct TcGeomArgs { int ks, jt; };
-
 // the digits of an integer (time4: of its square), lowest first
 template <int MODE>
 __device__ __forceinline__ void digits_of(float amp, float mean, int L, int s, short *d) {
@@ -257,7 +253,7 @@ __device__ bool four_digits(TimePlan &t, float vmax, int nx) {
 
 // CPT: window columns nxc + nx_corr - 1 (below 256 CPT) per thread
 template <int MODE, int CPT>
-__global__ void __launch_bounds__(TC_THREADS) k_tprep(Plan P, TcGeomArgs G) {
+__global__ void __launch_bounds__(TC_THREADS) k_tprep(Plan P) {
     using Tr = TcTraits<MODE>;
     using S = typename Tr::S;
     constexpr int WP = 256 * CPT, LMAX = MODE == 0 ? 2 : 4;
@@ -1043,9 +1039,10 @@ __global__ void __launch_bounds__(TC_THREADS) k_tpeak(Plan P) {
 // digits' three weights fit tensor memory (-time), else 64 (-time4: up to
 // seven weights); the widest slab whose operands fit shared memory.
 constexpr size_t SMEM_MAX = 227 * 1024;
+struct TcGeom { int ks, jt; };            // columns of the window per slab, lag columns per tile
 template <int MODE>
-TcGeomArgs tc_geom(const Plan &P) {
-    TcGeomArgs g;
+TcGeom tc_geom(const Plan &P) {
+    TcGeom g;
     g.jt = (MODE == 0 && P.nxc >= 128) ? 128 : 64;
     g.ks = std::min(P.nx_corr, g.jt);
     while (g.ks > 16 && tc_layout<MODE>(P.ny_corr, P.nyc, g.ks, g.jt).bytes > SMEM_MAX) g.ks >>= 1;
@@ -1064,12 +1061,12 @@ cudaError_t time_setup_t(const Plan &P) {
 }
 template <int MODE>
 void launch_tcorr_t(const Plan &P, cudaStream_t s) {
-    const TcGeomArgs g = tc_geom<MODE>(P);
+    const TcGeom g = tc_geom<MODE>(P);
     const int cpt = prep_cpt(P);
     const size_t psm = (size_t)8 * 256 * cpt * 8;
-    if (cpt == 1) k_tprep<MODE, 1><<<P.nwin, TC_THREADS, psm, s>>>(P, g);
-    else if (cpt == 2) k_tprep<MODE, 2><<<P.nwin, TC_THREADS, psm, s>>>(P, g);
-    else k_tprep<MODE, 4><<<P.nwin, TC_THREADS, psm, s>>>(P, g);
+    if (cpt == 1) k_tprep<MODE, 1><<<P.nwin, TC_THREADS, psm, s>>>(P);
+    else if (cpt == 2) k_tprep<MODE, 2><<<P.nwin, TC_THREADS, psm, s>>>(P);
+    else k_tprep<MODE, 4><<<P.nwin, TC_THREADS, psm, s>>>(P);
     const dim3 grid(((P.nyc + 127) / 128) * (P.nxc / g.jt), P.nwin);
     const size_t sm = tc_layout<MODE>(P.ny_corr, P.nyc, g.ks, g.jt).bytes;
     if constexpr (MODE == 0) {
