@@ -520,9 +520,10 @@ int ctx_batch_windows(const xcg_ctx *c, int nlocs, int strip_len) {
     // their kernels fill the GPU to a half or less and overlap well (144 windows of
     // 64 x 64 60 -> 54 us, 192 of 256 x 256 540 -> 457, through host buffers 200 of
     // 128 x 128 321 -> 269; over 70 grids of this range 0.97 to 1.21, most 1.04 to
-    // 1.14).  Fewer windows lose in the launches and in shared rows (40 of 128 x 128:
-    // 61 against 63 us), smaller ones too (120 of 64 x 64, 1.9 million pixels: 52
-    // against 60); 400 to 511 measured from 0.96 to 1.03.
+    // 1.14; 300 to 384 windows 1.01 to 1.10 over 20 more).  Fewer windows lose in the
+    // launches and in shared rows (40 of 128 x 128: 61 against 63 us), smaller ones
+    // too (120 of 64 x 64, 1.9 million pixels: 52 against 60); 400 to 511 measured
+    // from 0.96 to 1.09.
     // Neither these nor the time modes' two batches cut a strip: the last window
     // before a cut does not see the next one's first value.
     int bw = c->max_batch;
@@ -532,8 +533,8 @@ int ctx_batch_windows(const xcg_ctx *c, int nlocs, int strip_len) {
     const bool few = freq && B.rc && !B.tc_form && whole && nlocs >= 96 && nlocs <= 384 &&
                      (size_t)nlocs * B.npx * B.npy >= ((size_t)1 << 21);
     const bool many = freq && nlocs >= 512 && (B.tc_form || B.rc);
-    // The time modes from 400 windows on (1.01 to 1.10 over ten grids; 200 to 300:
-    // 0.98 to 1.04), -time4 up to 64 x 128 windows (128 x 128 gain nothing, 600 of them
+    // The time modes from 400 windows on (1.01 to 1.10 over 35 grids; 200 to 300:
+    // 0.98 to 1.04, 340 to 380 1.00 to 1.19), -time4 up to 64 x 128 windows (128 x 128 gain nothing, 600 of them
     // 8.60 against 8.55 ms, and lose where the integer kernel takes windows, 13.7
     // against 15.2).
     const bool time = !freq && whole && nlocs >= 400 && (B.corr_mode == 0 || B.nx_corr * B.ny_corr <= 64 * 128);
