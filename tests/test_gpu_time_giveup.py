@@ -16,13 +16,14 @@ def test_a_wait_that_runs_out_leaves_the_window_to_the_integer_kernel(xs, ys, mo
     locs = xg.grid(nx, ny, 4, 6, xs, ys)
     with xg.Context(xg.params(xs, ys, corr_mode=mode)) as ctx:
         ctx.set_profiling(True)
-        ctx.correlate(m, s, locs, strip_len=4)
-        usual = ctx.correlate(m, s, locs, strip_len=4)
-        ms = ctx.stats().kernel_ms[1]
+        ms = []
+        for _ in range(4):
+            usual = ctx.correlate(m, s, locs, strip_len=4)
+            ms.append(ctx.stats().kernel_ms[1])
         ctx.inject_stage_timeout()
         given_up = ctx.correlate(m, s, locs, strip_len=4)
         if (xs, ys, mode) != (128, 64, 1):                   # (too bright for digits: the integer kernel's either way)
-            assert ctx.stats().kernel_ms[1] > 1.2 * ms       # both kernels took every window
+            assert ctx.stats().kernel_ms[1] > 1.2 * min(ms)  # both kernels took every window
         after = ctx.correlate(m, s, locs, strip_len=4)
     assert not (usual["flags"] & xg.FLAG_STAGE_TIMEOUT).any()
     assert given_up.tobytes() == usual.tobytes() and after.tobytes() == usual.tobytes()
