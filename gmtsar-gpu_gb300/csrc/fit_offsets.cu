@@ -284,13 +284,14 @@ struct FitCall {
 template <int CTAS>
 cudaError_t launch_fit(const FitCall &f, bool ask, bool &ran) {
     ran = false;
-    // the kernel's attributes, per device (idempotent: every call may set them)
-    cudaError_t e = CTAS > 8 ? cudaFuncSetAttribute(k_fit<CTAS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) : cudaSuccess;
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_fit<CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fit_smem(FIT_KEEP));
-    if (e != cudaSuccess) return e;
     const long long per = (long long)CTAS * FIT_THREADS;           // points a cluster takes at a time
     const int keep = (int)std::min<long long>(FIT_KEEP, (f.n + per - 1) / per * FIT_THREADS);
+    // the kernel's attributes, per device (idempotent: every call may set them);
+    // up to 46 KB need none
+    cudaError_t e = CTAS > 8 ? cudaFuncSetAttribute(k_fit<CTAS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) : cudaSuccess;
+    if (e == cudaSuccess && fit_smem(keep) > 46 * 1024)
+        e = cudaFuncSetAttribute(k_fit<CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fit_smem(FIT_KEEP));
+    if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * CTAS);
     cfg.blockDim = dim3(FIT_THREADS);

@@ -408,9 +408,13 @@ def fit_offsets(d_results: int, d_locs: int, nlocs: int, d_out: int, ri=2, x_off
     device result array; d_out is a device buffer of sizeof(Fit) bytes.  ctas:
     16, 8 or 1 CTAs per axis (xcg_debug_fit_offsets), 0 the most that fit."""
     L = load()
-    args = (d_results, d_locs, int(nlocs), int(ri), int(x_offset), int(y_offset), float(astretcha), float(snr_min),
-            int(npar_range), int(npar_azimuth), int(robust_iters), d_out, stream)
-    _check(L.xcg_debug_fit_offsets(int(ctas), *args) if ctas else L.xcg_fit_offsets(*args))
+    if ctas:
+        _check(L.xcg_debug_fit_offsets(int(ctas), d_results, d_locs, int(nlocs), int(ri), int(x_offset), int(y_offset),
+                                       float(astretcha), float(snr_min), int(npar_range), int(npar_azimuth),
+                                       int(robust_iters), d_out, stream))
+        return
+    _check(L.xcg_fit_offsets(d_results, d_locs, int(nlocs), int(ri), int(x_offset), int(y_offset), float(astretcha),
+                             float(snr_min), int(npar_range), int(npar_azimuth), int(robust_iters), d_out, stream))
 
 
 def tc_gemm_check(m_tiles: int, n_tile: int, k: int, n_total: int, d_a: int, d_b: int, d_c: int, stream: int = 0):
