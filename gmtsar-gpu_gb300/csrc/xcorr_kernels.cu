@@ -1089,10 +1089,12 @@ static size_t cols_smem(int) {
 // only wait (100 windows of 64 x 64: 14.3 -> 18.4 us).  The most windows of a
 // batch, alone and with another batch of its call in flight, by the transform's
 // length, from whole calls with and without clusters (us):
-//   up to 256 points  152 alone: 152 of 128 x 128 151 against 154.  100 beside
-//                     another: 200 in two batches 172 against 177; 300 in two 217
-//                     against 216, and from four contexts at once 204 against 187
-//                     (195 before there were clusters)
+//   up to 256 points  152 alone: 152 of 128 x 128 151 against 154.  Beside another
+//                     152 where every team has two row pairs or more (250 of 128 x
+//                     256 in two batches 256 against 268, 300 344 against 346), 100
+//                     where it has one: 200 of 128 x 128 172 against 177; 240 158
+//                     against 160, but from four contexts at once 139 against 127
+//                     (130 before there were clusters)
 //   512               152 both: 152 of 256 x 256 327 against 367, 300 in two batches
 //                     495 against 505
 //   1024 (one CTA     72 alone: 72 of 512 x 128 305 against 312, 76 317 against 315,
@@ -1100,7 +1102,13 @@ static size_t cols_smem(int) {
 //                     against 303, 76 308 against 308, 120 360 against 344
 constexpr int PEAK_CL = 4;
 template <int N>
-constexpr int peak_cl_windows(bool alone) { return N <= 256 ? (alone ? 152 : 100) : N <= 512 ? 152 : (alone ? 72 : 38); }
+static bool peak_cluster(const Plan &P) {
+    const int pairs = P.nyc / 2 / (PEAK_CL * (256 / fft_lanes(N)));      // row pairs of a team
+    if (pairs == 0 || P.peak_cfg != 0) return false;
+    const bool alone = P.batches <= 1;
+    const int most = N <= 256 ? (alone || pairs > 1 ? 152 : 100) : N <= 512 ? 152 : (alone ? 72 : 38);
+    return P.nwin <= most;
+}
 // resident k_peak CTAs per SM for configuration cfg
 template <int N>
 constexpr int peak_minb(int cfg) { return (N <= 256) ? (cfg == 1 ? 3 : 4) : (N <= 512 ? (cfg == 1 ? 2 : 3) : 1); }
@@ -1209,7 +1217,7 @@ static void launch_cols_t(const Plan &P, cudaStream_t s) {
 }
 template <int N>
 static void launch_peak_t(const Plan &P, cudaStream_t s) {
-    if (P.nwin <= peak_cl_windows<N>(P.batches <= 1) && P.nyc / 2 >= PEAK_CL * (256 / fft_lanes(N)) && P.peak_cfg == 0) {
+    if (peak_cluster<N>(P)) {
         launch_chain(P, k_peak<N, peak_minb<N>(0), 256, PEAK_CL>, dim3(P.nwin * PEAK_CL), 256, peak_smem<N>(), s, PEAK_CL);
         return;
     }

@@ -9,7 +9,7 @@ from xcorr_gb300 import synth
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("xs,ys,n", [(64, 64, 152), (64, 64, 153), (64, 64, 200), (64, 64, 202), (32, 64, 30), (128, 128, 9),
+@pytest.mark.parametrize("xs,ys,n", [(64, 64, 152), (64, 64, 153), (64, 64, 200), (64, 64, 202), (64, 128, 202), (64, 128, 306), (32, 64, 30), (128, 128, 9),
                                      (128, 32, 152), (128, 32, 153), (256, 64, 72), (256, 64, 73), (256, 32, 76), (256, 32, 78),
                                      (256, 16, 5)])
 def test_cluster_and_single_cta(xs, ys, n):
