@@ -249,9 +249,10 @@ xcg_status xcg_set_row_sharing(xcg_ctx *ctx, int32_t enable);
  * 512-point transforms, one for 1024), one per window, or a cluster of four per
  * window in batches of up to 152 windows (72 for 1024 points; beside another
  * batch of the call 38 for 1024 and, up to 256 points, 100 where a team of the
- * cluster has one row pair) where the surface has a row pair for every team; 1 always one CTA per window, one fewer
- * per SM where 0 has several; 2 one CTA of 512 threads per window (transforms up
- * to 512 points; for 1024 one of 256).  Every shape gives the same bits. */
+ * cluster has one row pair) where the surface has a row pair for every team; 1
+ * always one CTA per window, one fewer per SM where 0 has several; 2 one CTA of
+ * 512 threads per window (transforms up to 512 points; for 1024 one of 256).
+ * Every shape gives the same bits. */
 xcg_status xcg_set_launch_shapes(xcg_ctx *ctx, int32_t cols_cfg, int32_t peak_cfg);
 
 /* Split each later call's windows into this many batches (whole strips; at
