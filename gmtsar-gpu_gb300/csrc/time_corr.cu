@@ -49,7 +49,7 @@ constexpr int RI = 2, RJ = 4;
 // not ended by the limit of a second wait either (the record says so).
 struct TimePlan {
     long long d2;          // sum of b*b (time4: of v*v, modulo 2^64)
-    int limbs, shift, rows, failed;
+    int limbs, failed, shift, rows;      // (k_tcorr reads the first two at once)
 };
 // A window's amplitudes: the master patch (rows of npx) and the slave's centre
 // (row stride a2s), its own or rows of its chunks of shared row segments
@@ -839,7 +839,8 @@ __global__ void __launch_bounds__(TC_THREADS) k_tcorr(Plan P) {
 #pragma unroll 1
     for (int item = blockIdx.x; item < P.nwin * tiles; item += gridDim.x) {
         const int w = item / tiles, t0 = item - w * tiles;
-        if (time_plan(P, w)->limbs != 0 && time_plan(P, w)->failed == 0) continue;      // formed on the tensor cores
+        const int2 lf = *reinterpret_cast<const int2 *>(&time_plan(P, w)->limbs);
+        if (lf.x != 0 && lf.y == 0) continue;                            // formed on the tensor cores
         const int i0 = (t0 / tiles_j) * TI, j0 = (t0 % tiles_j) * TJ;    // first lag row and column of the tile
         const float m1f = (float)P.means[2 * w], m2f = (float)P.means[2 * w + 1];
         const TimeAmps amps = time_amps(P, w);
